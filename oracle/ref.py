@@ -16,10 +16,16 @@ import numpy as np
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "_ref", "libchanref.so")
-# the reference sources: CHANFAST_REFERENCE_SRC, else a checkout named
-# `reference` beside this repository
-REFERENCE_SRC = os.environ.get("CHANFAST_REFERENCE_SRC") or os.path.abspath(
-    os.path.join(HERE, "..", "..", "reference"))
+
+
+def _source_dir():
+    """The reference sources: CHANFAST_REFERENCE_SRC, else a checkout named
+    `reference` beside this repository; "" when no sources are there."""
+    d = os.environ.get("CHANFAST_REFERENCE_SRC") or os.path.abspath(os.path.join(HERE, "..", "..", "reference"))
+    return d if os.path.isfile(os.path.join(d, "chanfast.c")) else ""
+
+
+REFERENCE_SRC = _source_dir()
 
 _lock = threading.Lock()
 _lib = None
@@ -38,7 +44,7 @@ class RefParams(ctypes.Structure):
 def build(quiet=True):
     """Compile oracle/_ref from the reference sources (needs the reference tree)."""
     if not os.path.isdir(REFERENCE_SRC):
-        raise FileNotFoundError(f"reference sources not found at {REFERENCE_SRC}")
+        raise FileNotFoundError("reference sources not found (set CHANFAST_REFERENCE_SRC)")
     subprocess.run(["make", "-C", HERE, f"REF={REFERENCE_SRC}", "-j8"], check=True,
                    stdout=subprocess.DEVNULL if quiet else None)
 
