@@ -164,10 +164,11 @@ int cf_device_field(cf_instance *inst, int field, double **dev_ptr, long long *n
 /* Run nsub substeps with CUDA events between the kernel groups on the
  * instance stream and return the summed device time of each group (ms) in
  * ms[CF_NKERNEL_GROUPS], in this order:
- *   0 ghosts (apply_bc), 1 rhs with the forward sweeps of the implicit
- *   solves, 2 back substitution of u, v, c and w (one launch), 3 mass-flux
- *   control u, 4 scalar-mean control c, 5 divergence + x FFT, 6 y FFT,
- *   7 Poisson, 8 inverse y FFT, 9 inverse x FFT, 10 projection.
+ *   0 ghosts (apply_bc), 1 rhs (on planes that fill the GPU with the forward
+ *   sweeps of the implicit solves), 2 line solves of u, v, c and w (one
+ *   launch), 3 mass-flux control u (with c's where one launch does both),
+ *   4 scalar-mean control c, 5 divergence + x FFT, 6 y FFT, 7 Poisson,
+ *   8 inverse y FFT, 9 inverse x FFT, 10 projection.
  * With power-of-two ny the y transforms run inside the Poisson launch
  * (k_poisson_fft): groups 6 and 8 are then empty and 7 holds all three.
  * Synchronises after every substep (timing only). */
@@ -245,8 +246,8 @@ int cf_batch_destroy(cf_batch *batch);
 
 /* ------------------------------------------------------------------------
  * Launch-shape autotuning.  Three kernels run with any of a few block shapes
- * and give the same results bit for bit: the back substitution (columns per
- * block: 64, 128), the Poisson / spectral Helmholtz band solve (column
+ * and give the same results bit for bit: the line solves (columns per block,
+ * or threads of a partitioned block's columns: 64, 128), the Poisson / spectral Helmholtz band solve (column
  * pairs per block: 64, 128) and the projection (block of j by i: 32x2, 32x4,
  * 32x8, 64x2).  cf_create times the candidates on the new instance (before
  * it holds state) and keeps the fastest; cf_batch_create does the same on

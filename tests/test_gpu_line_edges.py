@@ -1,0 +1,50 @@
+"""Substeps at the sizes where the line solves, the right-hand side's row blocks
+and the packed x transforms change form, against the numpy restatement:
+
+* k_line's chunks of 16 rows: one short chunk, exactly full ones, a last chunk
+  of one row (where w, one row shorter, has none), the tallest partitioned
+  column (192 rows) and the first whole-column one (193);
+* planes whose columns do not fill the last group of 16 (or of 32), odd and even;
+* x transforms of two columns each: an odd last column, 16-column blocks with
+  one column and with fifteen.
+
+Bars as test_gpu_parity.py: relative L2 1e-13 on u, v, w, c and 1e-10 on p
+(rounding of u* by 1e-16 is divided by dt and passes the inverse Laplacian),
+1e-9 of the column scale on the log, and for the two control values at least
+1e-14 / dt."""
+import numpy as np
+import pytest
+
+import chanfast_np as cn
+import ic
+
+pytestmark = pytest.mark.gpu
+
+CASES = [(2, 12, 15, 4), (4, 10, 9, 6), (2, 16, 18, 15), (4, 15, 81, 16), (2, 9, 16, 17), (4, 8, 25, 17),
+         (4, 12, 30, 32), (2, 15, 45, 33), (4, 20, 6, 49), (4, 6, 5, 192), (2, 6, 5, 193), (4, 8, 10, 193)]
+
+
+@pytest.mark.parametrize("order,nx,ny,nz", CASES)
+def test_substeps_match_restatement(cf, gpu, order, nx, ny, nz):
+    prm = cn.Params(order=order, nx=nx, ny=ny, nz=nz, lx=2 * np.pi, ly=np.pi, lz=2.0, dt=1e-3, nu=1.0 / 3000.0,
+                    prandtl=0.71, setuframe=0.3, betg_x=0.1, betg_y=0.05, betg_z=0.02)
+    g = cn.Grid(prm)
+    u, v, w, c = ic.raw_state(prm, g.dz, 11, 0.1, 0.01)
+    cn.project_initial(u, v, w, prm, g, 1.0)
+    st = cn.new_state(u, v, w, c, g)
+    with cf.Instance(cf.Config.from_params(prm)) as inst:
+        for nm, a in zip("uvwc", (u, v, w, c)):
+            inst.set_field(nm, a)
+        inst.step(4)
+        inst.sync()
+        cn.run(st, prm, g, 4)
+        I = (slice(3, 3 + nx), slice(3, 3 + ny), slice(3, 3 + nz))
+        for nm in "uvwcp":
+            a, b = inst.get_field(nm)[I], getattr(st, nm)[I]
+            rel = np.linalg.norm(a - b) / np.linalg.norm(b)
+            assert rel <= (1e-10 if nm == "p" else 1e-13), (nm, rel)
+        log, ref = inst.log(), np.array(st.log)
+        assert log.shape == ref.shape
+        bar = 1e-9 * np.maximum(np.abs(ref).max(axis=0), 1e-3)
+        bar[[0, 5]] = np.maximum(bar[[0, 5]], 1e-14 / prm.dt)
+        assert np.all(np.abs(log - ref) <= bar), np.abs(log - ref).max(axis=0)

@@ -30,22 +30,21 @@ struct WallRowsD {
 // (instance.cu, cf_tune) times the candidates and keeps the fastest; the
 // defaults are the hand-picked shapes.  Results do not depend on the choice:
 // these kernels index their work from blockDim, one column (pair, point) per
-// thread, and the per-warp row sums of k_back4 cover the same 32 columns
-// whatever the block size.
+// thread, and the column sums of k_line cover the same columns whatever the
+// block size.
 struct LaunchShape {
-    int solve_threads = 128;           // k_back4: columns per block (64, 128)
+    int solve_threads = 128;           // k_line: columns per block of the back sweep (64, 128), threads of the
+                                       // partitioned solve (line_threads)
     int pois_threads = 128;            // k_poisson / k_helmholtz_spectral: column pairs per block (64, 128)
     int proj_bx = 32, proj_by = 4;     // k_project block: j by i (32x2, 32x4, 32x8, 64x2)
 };
-// k_back4 is bound to 128 threads: a 256-thread bound costs it 4 registers
-// and one resident block per SM (measured 40 % slower)
-constexpr int SOLVE_THREADS_MAX = 128;
 constexpr int POIS_THREADS_MAX = 128;
 constexpr int PROJ_THREADS_MAX = 256;
 
 // Geometry / metric tables shared by all kernels of an instance.
 struct Geo {
     LaunchShape shape;    // tuned launch shapes (host side; kernels read blockDim)
+    bool partitioned;     // line solves partitioned, k_rhs without the forward sweeps (line_partitioned)
     int order, nx, ny, nz, n2, nkx;
     long long plane;      // nx*ny (points per k-plane)
     long long splane;     // nkx*ny (spectral columns per k-plane)
@@ -65,20 +64,32 @@ struct Geo {
     double idx, idy;      // 1/dx, 1/dy
 };
 
-// Line-solve factorisation on device (see host_band.h LineFactor).
-struct FactorD {
-    int k0, n;
-    const double *F1, *F2, *F3, *DEN, *P, *Q, *R;
-};
+// Line solves (k_line, kernels_solve.cu).  Partitioned: a column's rows are cut
+// into chunks of LINE_R rows, one thread per chunk and two columns.
+constexpr int LINE_R = 16;
+constexpr int LINE_MAX_ROWS = 192;        // 12 chunks (line_partitioned)
+constexpr int LINE_STATS = 11;            // column sums of k_line that the controls read
+constexpr int CONTROL_THREADS = 512;
+__host__ __device__ constexpr int line_chunk_count(int nz) { return (nz + LINE_R - 1) / LINE_R; }
+// doubles of a chunk's recurrence rows, one 16-byte slot more so that the
+// chunks of a warp read different banks, and of a boundary matrix
+__host__ __device__ constexpr int line_chunk_stride(int order) { return LINE_R * (order == 2 ? 2 : 6) + 2; }
+__host__ __device__ constexpr int line_mat_stride(int order) { return order == 2 ? 1 : 10; }
+// column pairs that a block of `threads` threads takes at C chunks: 8 a group
+// of 16 columns
+__host__ __device__ constexpr int line_lanes(int threads, int C) { return 8 * (threads / (8 * C)); }
 
-// Back substitution of one implicit solve (its forward sweep runs in k_rhs).
+// One line solve: A x = h per column.
 struct SolveArgs {
     double* x;            // field: out, the new value (all n2 rows)
-    const double* s;      // forward-substituted vector, rows k0 .. k0+n-1
-    FactorD fac;          // back-substitution multipliers P, Q, R; rows k0 .. k0+n-1
+    const double* s;      // right-hand side as k_rhs leaves it (partitioned: h; else forward-swept), rows GZ .. GZ+n-1
+    const double* rows;   // line_rows table (partitioned)
+    const double* back;   // back_rows table (the back sweep alone)
+    int n;                // rows
     double bc_bot, bc_top;
     WallRowsD bcb, bct;   // apply_bc closure rows for this field
-    double* partial;      // per-warp row sums [nwarps][n2] or null
+    double* partial;      // column sums [LINE_STATS][ngroups] per group of columns, or null
+    long long ngroups;
 };
 
 struct FftPlan {
@@ -97,12 +108,13 @@ struct GhostArgs {
     double bc_u, bc_v, bc_c_bot, bc_c_top, bc_w;
 };
 
-// Forward sweep of one implicit solve, fused into k_rhs (see host_band.h
-// fused_rows): s_i = sum cu_m x_{k+m} + cf f_k + cg g_k + c0 - f1 s_{i-1} - ...
-struct FwdSweep {
-    double* g;             // in: previous-stage RHS g; out: the forward-substituted s (same rows)
+// Right-hand side of one implicit solve, formed in k_rhs (see host_band.h
+// fused_rows): h_k = sum cu_m x_{k+m} + cf f_k + cg g_k + c0, and with the
+// forward sweep s_k = h_k - f1 s_{k-1} - f2 s_{k-2} - f3 s_{k-3}
+struct HelmRhs {
+    double* g;             // in: previous-stage RHS g; out: h or s (same rows)
     const double* gshift;  // device scalar added to g (mass-flux lazily applied), or null
-    const double* rows;    // fused forward rows [n][fused_width]
+    const double* rows;    // fused rows [n][fused_width]
 };
 
 struct RhsArgs {
@@ -110,9 +122,10 @@ struct RhsArgs {
     double *fu, *fv, *fw, *fc;
     double nu, kappa;              // nu and nu/prandtl
     double betg_x, betg_y, betg_z;
-    FwdSweep sw[4];                // u, v, w, c
+    HelmRhs sw[4];                 // u, v, w, c
     WallRowsD wbot, wtop;          // apply_bc_w closure rows (ghost values of the old w)
     double wbc_bot, wbc_top;
+    int chunk;                     // rows per block (rhs_chunk); all of them with the forward sweeps
 };
 
 struct MassArgs {
@@ -133,12 +146,14 @@ struct MassArgs {
     double* nonfinite;    // device flag: set to 1 when the bulk mean or the control is NaN / Inf
 };
 
-struct RowAvgArgs {
-    const double* partial;   // per-warp row sums [nwarps][n2]
-    long long nwarps;
-    int n2;
-    double scale;            // 1 / (nx ny)
-    double* avg;             // [n2] out
+// Both controls of a z-implicit substep from k_line's column sums.
+struct ControlArgs {
+    MassArgs m[2];             // u, c (their avg is not read)
+    const double* partial[2];  // column sums [LINE_STATS][ngroups] of u and c
+    long long ngroups;
+    double scale, ilz;         // 1 / (nx ny), 1 / sum of dz
+    double* sums;              // [2][LINE_STATS] device scratch
+    unsigned* ticket;          // blocks done, 0 between launches
 };
 
 struct DivArgs {
@@ -234,12 +249,12 @@ struct ProjArgs {
 // otherwise as apply_bc_w leaves them (after the spectral solves)
 void launch_ghosts(const Geo& G, const GhostArgs& A, cudaStream_t st, bool extrap = true);
 void launch_rhs(const Geo& G, const RhsArgs& A, bool implicit3d, cudaStream_t st);
-// k_back4 block: one thread per column, LaunchShape::solve_threads per block
 struct SolveBatch {
     SolveArgs a[4];   // u, v, c, w
 };
-void launch_back4(const Geo& G, const SolveBatch& B, cudaStream_t st);
-void launch_mass(const Geo& G, const double* partial, double* avg, const MassArgs& M, cudaStream_t st);
+void launch_line(const Geo& G, const SolveBatch& B, cudaStream_t st);
+long long line_groups(const Geo& G);
+void launch_control(const ControlArgs& A, cudaStream_t st);
 void launch_mass_control(const MassArgs& M, cudaStream_t st);
 void launch_div_fftx(const Geo& G, const DivArgs& A, cudaStream_t st);
 bool fftx_batched_supported(int nx);
@@ -257,8 +272,13 @@ cudaError_t fft_set_smem_limits(int max_n);
 // ------------------------------------------------- batched launches (batch.cuh)
 struct BatchLaunch;
 dim3 grid_ghosts(const Geo& G);
-dim3 grid_rhs(const Geo& G);
-dim3 grid_back4(const Geo& G);
+dim3 grid_rhs(const Geo& G, int chunk);
+constexpr int RHS_MIN_ROWS = 6;      // fewest rows of a k_rhs block (its wall closures reach two rows)
+long long rhs_tiles(const Geo& G);
+int rhs_chunk(const Geo& G, int sms, bool sweep);
+int line_threads(const Geo& G);
+dim3 grid_line(const Geo& G);
+size_t line_smem(const Geo& G);
 dim3 grid_div(const Geo& G);                       // power-of-two nx: divergence
 dim3 grid_r2c(const Geo& G, int nrows, int nfields);
 dim3 grid_div_fftx(const Geo& G);                  // other nx: divergence + x transform
@@ -267,12 +287,10 @@ dim3 grid_poisson(const Geo& G);
 dim3 grid_c2r(const Geo& G, int nrows, int nfields);
 dim3 grid_project(const Geo& G);
 bool batch_pow2(int n);                            // n has a power-of-two transform kernel
-RowAvgArgs row_average_args(const Geo& G, const double* partial, double* avg);
 void launch_ghosts_batch(const BatchLaunch& L, int order, cudaStream_t st);
 void launch_rhs_batch(const BatchLaunch& L, int order, cudaStream_t st);
-void launch_back4_batch(const BatchLaunch& L, int order, cudaStream_t st);
-void launch_row_average_batch(const BatchLaunch& L, cudaStream_t st);
-void launch_mass_control_batch(const BatchLaunch& L, cudaStream_t st);
+void launch_line_batch(const BatchLaunch& L, int order, cudaStream_t st);
+void launch_control_batch(const BatchLaunch& L, cudaStream_t st);
 void launch_div_batch(const BatchLaunch& L, int order, cudaStream_t st);
 void launch_r2c_batch(const BatchLaunch& L, int nx, cudaStream_t st);
 void launch_div_fftx_batch(const BatchLaunch& L, int order, int nx, cudaStream_t st);

@@ -541,6 +541,65 @@ std::vector<double> fused_rows(const Metrics& m, const ImplicitSet& s, bool is_w
     return rows;
 }
 
+std::vector<double> back_rows(const LineFactor& L, int order)
+{
+    const int H = order == 2 ? 1 : 3;
+    std::vector<double> t((size_t) L.n * H);
+    for (int i = 0; i < L.n; i++) {
+        t[(size_t) i * H] = L.P[i];
+        if (H == 3) {
+            t[(size_t) i * H + 1] = L.Q[i];
+            t[(size_t) i * H + 2] = L.R[i];
+        }
+    }
+    return t;
+}
+
+std::vector<double> line_rows(const LineFactor& L, int order, int chunks, int R, int stride, int mstride)
+{
+    const int H = order == 2 ? 1 : 3, n = L.n;
+    const double* F[3] = {L.F1.data(), L.F2.data(), L.F3.data()};
+    const double* B[3] = {L.P.data(), L.Q.data(), L.R.data()};
+    const int C = chunks;
+    std::vector<double> t((size_t) C * (stride + 2 * mstride), 0.0);
+    for (int c = 0; c < C; c++) {
+        double* f = &t[(size_t) c * stride];
+        double* b = f + R * H;
+        for (int r = 0; r < R && c * R + r < n; r++)
+            for (int m = 0; m < H; m++) {
+                f[r * H + m] = F[m][c * R + r] / L.DEN[c * R + r];
+                b[r * H + m] = B[m][c * R + r];
+            }
+        if (chunks < 2) continue;
+        // column m of the boundary matrices: both recurrences from a unit
+        // value m + 1 rows outside the chunk, to its last (first) H rows
+        double* Mf = &t[(size_t) C * stride + (size_t) c * mstride];
+        double* Mb = Mf + (size_t) C * mstride;
+        for (int m = 0; m < H; m++) {
+            double v[3] = {0.0, 0.0, 0.0}, w[3] = {0.0, 0.0, 0.0};   // the last H values, newest first
+            v[m] = w[m] = 1.0;
+            for (int r = 0; r < R; r++) {
+                double s = 0.0, y = 0.0;
+                for (int q = 0; q < H; q++) {
+                    s -= f[r * H + q] * v[q];
+                    y -= b[(R - 1 - r) * H + q] * w[q];
+                }
+                for (int q = H - 1; q > 0; q--) {
+                    v[q] = v[q - 1];
+                    w[q] = w[q - 1];
+                }
+                v[0] = s;
+                w[0] = y;
+            }
+            for (int q = 0; q < H; q++) {
+                Mf[q * H + m] = v[q];
+                Mb[q * H + m] = w[q];
+            }
+        }
+    }
+    return t;
+}
+
 std::vector<double> channel_rows(const Metrics& m, const ImplicitSet& s, bool is_w, double nuadt,
                                  double gamdt, double zetdt)
 {

@@ -93,8 +93,10 @@ ImplicitSet make_implicit_u(const Metrics& m, double nubdt, double gamdt, double
                             double bc_top, double kappa, bool want_green);
 ImplicitSet make_implicit_w(const Metrics& m, double nubdt, double bc_bot, double bc_top);
 
-// Per-row coefficients of the fused forward sweep used on the device:
-//   s_i = sum_m cu_m x_{k+m} + cf f_k + cg g_k + c0 - f1 s_{i-1} - f2 s_{i-2} - f3 s_{i-3}
+// Per-row coefficients of the scaled right-hand side of a line solve and of
+// its forward sweep:
+//   h_i = sum_m cu_m x_{k+m} + cf f_k + cg g_k + c0
+//   s_i = h_i - f1 s_{i-1} - f2 s_{i-2} - f3 s_{i-3}
 // which is, up to rounding, ((H(nuadt) x + gamdt f + zetdt g - hbc) dvol - F.s) / DEN
 // (chanfast.c:469-482 with the forward half of tridag/heptdag).  Row i holds
 // [cu_{-H..H}, cf, cg, c0, f1, f2, f3] with H = 1 (order 2) or 3 (order 4).
@@ -102,11 +104,25 @@ std::vector<double> fused_rows(const Metrics& m, const ImplicitSet& s, bool is_w
                                double gamdt, double zetdt);
 inline int fused_width(int order) { return (order == 2 ? 3 : 7) + 6; }
 
+// Back recurrence of a line solve, row i: P (Q, R at order 4),
+// x_i = s_i - P x_{i+1} - Q x_{i+2} - R x_{i+3}.
+std::vector<double> back_rows(const LineFactor& L, int order);
+
+// Tables of the partitioned line solve (k_line): the n rows cut into `chunks`
+// chunks of R rows, the last one filled up with zero coefficients.  Chunk c at
+// [c stride]: R rows of the forward recurrence f_1..f_H, scaled by the pivot
+// (s_i = h_i - f_1 s_{i-1} - ..), then R rows of the back recurrence P, Q, R
+// (x_i = s_i - P x_{i+1} - ..).  Then two sets of H x H boundary matrices
+// (mstride apart), one per chunk: the recurrence's response at the chunk's
+// last (back: first) H rows, nearest to the next chunk first, to the H
+// values before (after) it.
+std::vector<double> line_rows(const LineFactor& L, int order, int chunks, int R, int stride, int mstride);
+
 // Per-row coefficients of the channel scheme's Helmholtz right-hand side
 // (channel.c:455-467 and its v, c, w counterparts), z part:
 //   h_k = sum_m cu_m x_{k+m} + cf f_k + cg g_k + c0
 // = x + nuadt d2x/dz2 + gamdt f + zetdt g - hbc; the device adds
-// nuadt (d2/dx2 + d2/dy2) x.  Same row layout as fused_rows, f1..f3 = 0.
+// nuadt (d2/dx2 + d2/dy2) x.  Same row layout as fused_rows.
 std::vector<double> channel_rows(const Metrics& m, const ImplicitSet& s, bool is_w, double nuadt,
                                  double gamdt, double zetdt);
 

@@ -4,9 +4,9 @@
 // the per-substep coefficient sets.  cf_step issues, per RK3 substep, the
 // kernel sequence that replaces the body of chanfast.c:395-656 (order 2) /
 // 1319-1580 (order 4):
-//   ghosts -> rhs -> solve u -> mass control u -> solve v -> solve c ->
-//   scalar-mean control c -> solve w -> divergence+x FFT -> y FFT ->
-//   Poisson -> inverse y FFT -> inverse x FFT -> projection
+//   ghosts -> rhs -> line solves of u, v, c, w -> flow-rate and scalar-mean
+//   control -> divergence+x FFT -> y FFT -> Poisson -> inverse y FFT ->
+//   inverse x FFT -> projection
 #include <algorithm>
 #include <array>
 #include <cmath>
@@ -399,9 +399,8 @@ std::vector<int> fft_radices(int n)
 }  // namespace
 
 struct SetOffsets {
-    size_t F1, F2, F3, DEN, P, Q, R, hbc, green, rows;
-    int k0, n;
-    WallRowsD bot, top;
+    size_t green, rows, line, back;   // Green's function, right-hand side rows, line_rows and back_rows tables
+    int n;
     double gstats[4];
 };
 
@@ -427,10 +426,12 @@ struct cf_instance {
     double* gbuf[4] = {nullptr, nullptr, nullptr, nullptr};
     double2* spec = nullptr;
     double* scratch = nullptr;
-    double* partial = nullptr;     // per-warp row sums of the u solve
-    double* partial_c = nullptr;   // and of the c solve
-    double* avg = nullptr;
-    double* avg_c = nullptr;        // channel scheme: xy-average of c (avg holds u's)
+    double* partial = nullptr;      // column sums of the u solve (LINE_STATS x line_groups)
+    double* partial_c = nullptr;    // and of the c solve
+    double* csum = nullptr;         // control sums [2][LINE_STATS], then the control's ticket
+    double* avg = nullptr;          // channel scheme: xy-averages of u
+    double* avg_c = nullptr;        // and of c
+    int rhs_rows = 0;               // rows per k_rhs block (rhs_chunk)
     double* dscal = nullptr;        // [0] mdpdx, [1] dcdt, [2] non-finite flag, [3] copy-wait fault flag
     // channel scheme with the fused Helmholtz solves: device records [3][4]
     // (substep set, field u v w c) of k_poisson_fft_batch without FILL
@@ -461,6 +462,25 @@ struct cf_instance {
 };
 
 namespace {
+
+// Whether an instance on its own runs its line solves partitioned (k_line does
+// both sweeps, k_rhs takes any number of rows a block) or with the forward
+// sweep in k_rhs, up whole columns, and k_line walking back down.  The
+// partition is for planes too small to give every SM a k_rhs tile: k_rhs then
+// gets its blocks from the rows, and k_line's threads walk 16 rows instead of
+// all.  Measured, k_rhs + k_line in us, partitioned against whole columns:
+//   order 2: 64^3 30 : 100, 128 x 128 x 96 96 : 162, 192 x 192 x 128 250 : 258
+//   order 4: 64^3 40 : 157, 128 x 128 x 96 136 : 241, 192 x 192 x 128 339 : 334
+// The line lies at three quarters of the SMs (192 x 192 has 144 tiles): from
+// there on the row blocks' start costs what the idle SMs cost, and work on
+// other streams, which fills those, is slowed (256 x 256 x 192 at order 4,
+// three instances at once: 8.54 against 8.32 ms).  Above 192 rows the carries
+// through the chunks cost more than the walk (512 x 512 x 384: 2880 against
+// 1480 us).  In a batch the other members fill the GPU: whole columns.
+bool line_partitioned(bool channel, const Geo& G, int sms)
+{
+    return !channel && G.nz <= LINE_MAX_ROWS && 4 * rhs_tiles(G) <= 3 * sms;
+}
 
 int check_config(const cf_config* c)
 {
@@ -496,14 +516,12 @@ int build_tables(cf_instance* I, double dt)
                       double zetdt) {
         so.rows = A.add(channel ? channel_rows(m, s, is_w, nuadt, gamdt, zetdt)
                                 : fused_rows(m, s, is_w, nuadt, gamdt, zetdt));
-        so.k0 = s.fac.k0;
         so.n = s.fac.n;
-        so.F1 = A.add(s.fac.F1); so.F2 = A.add(s.fac.F2); so.F3 = A.add(s.fac.F3);
-        so.DEN = A.add(s.fac.DEN); so.P = A.add(s.fac.P); so.Q = A.add(s.fac.Q); so.R = A.add(s.fac.R);
-        so.hbc = A.add(s.hbc);
+        so.line = I->geo.partitioned ? A.add(line_rows(s.fac, C.order, line_chunk_count(C.nz), LINE_R,
+                                                       line_chunk_stride(C.order), line_mat_stride(C.order)))
+                                     : 0;
+        so.back = channel ? 0 : A.add(back_rows(s.fac, C.order));
         so.green = A.add(s.green.empty() ? std::vector<double>(m.n2, 0.0) : s.green);
-        so.bot = to_dev(s.bot);
-        so.top = to_dev(s.top);
         std::memcpy(so.gstats, s.green_stats, sizeof(so.gstats));
     };
     double uf = C.setuframe, vf = C.setvframe;
@@ -612,17 +630,6 @@ int build_tables(cf_instance* I, double dt)
     return CF_OK;
 }
 
-FactorD factor_of(cf_instance* I, const SetOffsets& so)
-{
-    double* b = I->coef;
-    FactorD f;
-    f.k0 = so.k0;
-    f.n = so.n;
-    f.F1 = b + so.F1; f.F2 = b + so.F2; f.F3 = b + so.F3; f.DEN = b + so.DEN;
-    f.P = b + so.P; f.Q = b + so.Q; f.R = b + so.R;
-    return f;
-}
-
 PoissonArgs poisson_args(cf_instance* I, const PoissonOffsets& po, double pdt)
 {
     double* b = I->coef;
@@ -667,11 +674,8 @@ struct Sink {
     virtual void mark() { if (tl) tl->mark(st); }
     virtual void ghosts(const Geo& G, const GhostArgs& A) { launch_ghosts(G, A, st); }
     virtual void rhs(const Geo& G, const RhsArgs& A) { launch_rhs(G, A, false, st); }
-    virtual void back4(const Geo& G, const SolveBatch& B) { launch_back4(G, B, st); }
-    virtual void mass(const Geo& G, const double* partial, double* avg, const MassArgs& M)
-    {
-        launch_mass(G, partial, avg, M, st);
-    }
+    virtual void line(const Geo& G, const SolveBatch& B) { launch_line(G, B, st); }
+    virtual void control(const Geo&, const ControlArgs& A) { launch_control(A, st); }
     virtual void div_fftx(const Geo& G, const DivArgs& A) { launch_div_fftx(G, A, st); }
     virtual void ffty(const Geo& G, const FftyArgs& A, int nrows) { launch_ffty(G, A, nrows, st); }
     virtual void poisson(const Geo& G, const PoissonArgs& A) { launch_poisson(G, A, st); }
@@ -848,7 +852,7 @@ void enqueue_substep(cf_instance* I, Sink& K)
     K.ghosts(G, GA);
     K.mark();
 
-    // RHS + forward sweeps; set index of each f slot (u, v, w, c) among the
+    // RHS and the line solves' right-hand sides; set index of each f slot (u, v, w, c) among the
     // implicit-solve sets (u, v, c, w)
     // chanfast: x-y diffusion explicit in f with nu; channel: implicit, in
     // h with nu alpha dt (channel.c:450-458)
@@ -867,6 +871,7 @@ void enqueue_substep(cf_instance* I, Sink& K)
     R.wtop = I->bc_wt;
     R.wbc_bot = 0.0;
     R.wbc_top = 0.0;
+    R.chunk = I->rhs_rows;
     if (channel) {
         launch_rhs(G, R, true, K.st);
         K.mark();
@@ -889,23 +894,35 @@ void enqueue_substep(cf_instance* I, Sink& K)
         const bool is_w = q == 3;
         SolveArgs& S = SB.a[q];
         S.x = fields[q];
-        S.s = I->gbuf[fidx[q]];   // the forward sweep in k_rhs left s there
-        S.fac = factor_of(I, so);
+        S.s = I->gbuf[fidx[q]];   // k_rhs left the right-hand side there
+        S.rows = I->coef + so.line;
+        S.back = I->coef + so.back;
+        S.n = so.n;
         S.bc_bot = bcb[q];
         S.bc_top = bct[q];
         S.bcb = is_w ? I->bc_wb : I->bc_ub;
         S.bct = is_w ? I->bc_wt : I->bc_ut;
         S.partial = partial[q];
+        S.ngroups = line_groups(G);
     }
-    K.back4(G, SB);
+    K.line(G, SB);
     K.mark();
-    for (int q = 0; q < 4; q += 2) {   // mass-flux control (u), scalar-mean control (c)
-        // each control has its own average buffer, so batched stages of
-        // different instances and fields never share one
-        double* avg = q == 0 ? I->avg : I->avg_c;
-        K.mass(G, partial[q], avg, mass_args(I, s, q, avg));
-        K.mark();
-    }
+    // flow-rate (u) and scalar-mean (c) control
+    ControlArgs CA;
+    CA.m[0] = mass_args(I, s, 0, nullptr);
+    CA.m[1] = mass_args(I, s, 2, nullptr);
+    CA.partial[0] = I->partial;
+    CA.partial[1] = I->partial_c;
+    CA.ngroups = line_groups(G);
+    CA.scale = 1.0 / ((double) G.nx * (double) G.ny);
+    double lz = 0.0;
+    for (int k = GZ; k < GZ + G.nz; k++) lz += I->m.dz[k];   // get_z_avg (get.c:490-502)
+    CA.ilz = 1.0 / lz;
+    CA.sums = I->csum;
+    CA.ticket = reinterpret_cast<unsigned*>(I->csum + 2 * LINE_STATS);
+    K.control(G, CA);
+    K.mark();
+    K.mark();   // one launch does both: the c group stays empty
     pressure_sequence(I, I->pois[s], (RK3_ALP[s] + RK3_BET[s]) * dt, s, true, K);
     I->substep++;
 }
@@ -930,15 +947,14 @@ void enqueue_substep(cf_instance* I, Timeline* tl = nullptr)
 // ST_PSOLVE: y transforms and Poisson solve, per member either the three
 // separate launches or the fused one (the member's own choice, so that a
 // member's result does not depend on its neighbours in a batch)
-enum StageKind { ST_GHOSTS, ST_RHS, ST_BACK4, ST_MASS, ST_DIV, ST_PSOLVE, ST_C2R, ST_PROJECT };
+enum StageKind { ST_GHOSTS, ST_RHS, ST_LINE, ST_CONTROL, ST_DIV, ST_PSOLVE, ST_C2R, ST_PROJECT };
 
 struct BatchStage {
     int kind = -1;
     std::vector<BatchRec<GhostArgs>> ghosts;
     std::vector<BatchRec<RhsArgs>> rhs;
-    std::vector<BatchRec<SolveBatch>> back4;
-    std::vector<BatchRec<RowAvgArgs>> rowavg;
-    std::vector<BatchRec<MassArgs>> control;
+    std::vector<BatchRec<SolveBatch>> line;
+    std::vector<BatchRec<ControlArgs>> control;
     std::vector<BatchRec<DivArgs>> div;        // power-of-two nx: the divergence ...
     std::vector<BatchRec<R2cArgs>> r2c;        // ... then its x transform
     std::vector<BatchRec<DivArgs>> div_fftx;   // other nx: both in one kernel
@@ -1013,6 +1029,14 @@ int build_helm_records(cf_instance* I)
     return CF_OK;
 }
 
+// A member's geometry in a batch: its line solves are not partitioned there
+// (line_partitioned).
+Geo whole_columns(Geo G)
+{
+    G.partitioned = false;
+    return G;
+}
+
 struct BatchSink : Sink {
     std::vector<BatchStage> stages;
     size_t cursor = 0;
@@ -1034,16 +1058,25 @@ struct BatchSink : Sink {
     {
         next(ST_GHOSTS).ghosts.push_back(batch_rec(G, A, grid_ghosts(G)));
     }
-    void rhs(const Geo& G, const RhsArgs& A) override { next(ST_RHS).rhs.push_back(batch_rec(G, A, grid_rhs(G))); }
-    void back4(const Geo& G, const SolveBatch& B) override
+    void rhs(const Geo& G, const RhsArgs& A) override
     {
-        next(ST_BACK4).back4.push_back(batch_rec(G, B, grid_back4(G)));
+        const Geo W = whole_columns(G);
+        RhsArgs B = A;
+        B.chunk = G.nz;
+        next(ST_RHS).rhs.push_back(batch_rec(W, B, grid_rhs(W, B.chunk)));
     }
-    void mass(const Geo& G, const double* partial, double* avg, const MassArgs& M) override
+    void line(const Geo& G, const SolveBatch& A) override
     {
-        BatchStage& S = next(ST_MASS);
-        S.rowavg.push_back(batch_rec(G, row_average_args(G, partial, avg), dim3(G.n2)));
-        S.control.push_back(batch_rec(G, M, dim3(1)));
+        const Geo W = whole_columns(G);
+        SolveBatch B = A;
+        for (SolveArgs& S : B.a) S.ngroups = line_groups(W);
+        next(ST_LINE).line.push_back(batch_rec(W, B, grid_line(W)));
+    }
+    void control(const Geo& G, const ControlArgs& A) override
+    {
+        ControlArgs B = A;
+        B.ngroups = line_groups(whole_columns(G));
+        next(ST_CONTROL).control.push_back(batch_rec(G, B, dim3(2 * LINE_STATS)));
     }
     void div_fftx(const Geo& G, const DivArgs& A) override
     {
@@ -1087,7 +1120,7 @@ struct BatchSink : Sink {
     }
 };
 
-enum BatchKernel { BK_GHOSTS, BK_RHS, BK_BACK4, BK_ROWAVG, BK_CONTROL, BK_DIV, BK_R2C, BK_DIV_FFTX, BK_FFTY,
+enum BatchKernel { BK_GHOSTS, BK_RHS, BK_LINE, BK_CONTROL, BK_DIV, BK_R2C, BK_DIV_FFTX, BK_FFTY,
                    BK_POISSON, BK_PFFT, BK_C2R, BK_PROJECT };
 
 struct BatchOp {
@@ -1140,9 +1173,9 @@ void add_groups(BatchProgram& P, int kernel, const std::vector<BatchRec<Args>>& 
 
 // Block shape of a batched launch of a tuned kernel: every record of a batch
 // is recorded with the batch's one launch shape (record()).
-dim3 back4_block(const std::vector<BatchRec<SolveBatch>>& r)
+dim3 line_block(const std::vector<BatchRec<SolveBatch>>& r)
 {
-    return dim3(r.empty() ? 128 : r[0].G.shape.solve_threads);
+    return dim3(r.empty() ? 128 : line_threads(r[0].G));
 }
 dim3 poisson_block(const std::vector<BatchRec<PoissonArgs>>& r)
 {
@@ -1166,11 +1199,8 @@ void compile(const BatchSink& K, BatchProgram& P)
         switch (S.kind) {
         case ST_GHOSTS: add_groups(P, BK_GHOSTS, S.ghosts, order, none); break;
         case ST_RHS: add_groups(P, BK_RHS, S.rhs, order, none); break;
-        case ST_BACK4: add_groups(P, BK_BACK4, S.back4, order, none, back4_block(S.back4)); break;
-        case ST_MASS:
-            add_groups(P, BK_ROWAVG, S.rowavg, none, none);
-            add_groups(P, BK_CONTROL, S.control, none, none);
-            break;
+        case ST_LINE: add_groups(P, BK_LINE, S.line, order, none, line_block(S.line)); break;
+        case ST_CONTROL: add_groups(P, BK_CONTROL, S.control, none, none); break;
         case ST_DIV:
             add_groups(P, BK_DIV, S.div, order, none);
             add_groups(P, BK_R2C, S.r2c, keynx, none);
@@ -1205,9 +1235,8 @@ void run_program(const BatchProgram& P, cudaStream_t st)
         switch (op.kernel) {
         case BK_GHOSTS: launch_ghosts_batch(L, op.key, st); break;
         case BK_RHS: launch_rhs_batch(L, op.key, st); break;
-        case BK_BACK4: launch_back4_batch(L, op.key, st); break;
-        case BK_ROWAVG: launch_row_average_batch(L, st); break;
-        case BK_CONTROL: launch_mass_control_batch(L, st); break;
+        case BK_LINE: launch_line_batch(L, op.key, st); break;
+        case BK_CONTROL: launch_control_batch(L, st); break;
         case BK_DIV: launch_div_batch(L, op.key, st); break;
         case BK_R2C: launch_r2c_batch(L, op.key, st); break;
         case BK_DIV_FFTX: launch_div_fftx_batch(L, op.key % 1024, op.key / 1024, st); break;
@@ -1315,7 +1344,7 @@ struct cf_batch {
 // ====================================================================== tuner
 //
 // Launch-shape autotuner.  Three kernels run with any of a few block shapes
-// and give the same results (LaunchShape, engine.cuh): k_back4 (columns per
+// and give the same results (LaunchShape, engine.cuh): k_line (columns per
 // block), k_poisson / k_helmholtz_spectral (column pairs per block) and
 // k_project (2-D block).  The tuner captures one substep's arguments of those
 // stages, times every candidate shape of each kernel with CUDA events on the
@@ -1475,15 +1504,20 @@ int time_launch(cudaStream_t st, F launch, float& ms)
 // Arguments of the tuned stages of one substep.
 struct CaptureSink : Sink {
     Geo G{};
-    bool has_back4 = false, has_pois = false, has_proj = false;
-    SolveBatch back4_args{};
+    bool has_line = false, has_pois = false, has_proj = false;
+    SolveBatch line_args{};
     PoissonArgs pois_args{};
     ProjArgs proj_args{};
     void mark() override {}
     void ghosts(const Geo&, const GhostArgs&) override {}
     void rhs(const Geo&, const RhsArgs&) override {}
-    void back4(const Geo& g, const SolveBatch& B) override { G = g; back4_args = B; has_back4 = true; }
-    void mass(const Geo&, const double*, double*, const MassArgs&) override {}
+    void line(const Geo& g, const SolveBatch& B) override
+    {
+        G = g;
+        line_args = B;
+        has_line = true;
+    }
+    void control(const Geo&, const ControlArgs&) override {}
     void div_fftx(const Geo&, const DivArgs&) override {}
     void ffty(const Geo&, const FftyArgs&, int) override {}
     void poisson(const Geo& g, const PoissonArgs& A) override { G = g; pois_args = A; has_pois = true; }
@@ -1493,13 +1527,13 @@ struct CaptureSink : Sink {
 };
 
 // Fastest candidate of each tuned kernel; `run(kind, shape)` launches that
-// kernel once with the shape (kind 0 back4, 1 Poisson, 2 projection).
+// kernel once with the shape (kind 0 line solves, 1 Poisson, 2 projection).
 template <class Run>
-int tune_shapes(cudaStream_t st, bool with_back4, Run run, LaunchShape& best)
+int tune_shapes(cudaStream_t st, bool with_line, Run run, LaunchShape& best)
 {
     best = LaunchShape{};
     float bt = 1e30f, t = 0.0f;
-    if (with_back4) {
+    if (with_line) {
         for (int c : TUNE_SOLVE) {
             LaunchShape S = best;
             S.solve_threads = c;
@@ -1553,11 +1587,11 @@ int tune_instance(cf_instance* I)
     auto run = [&](int kind, const LaunchShape& sh) {
         Geo G = K.G;
         G.shape = sh;
-        if (kind == 0) launch_back4(G, K.back4_args, I->stream);
+        if (kind == 0) launch_line(G, K.line_args, I->stream);
         else if (kind == 1) launch_poisson(G, K.pois_args, I->stream);
         else launch_project(G, K.proj_args, I->stream);
     };
-    int rc = tune_shapes(I->stream, K.has_back4, run, S);
+    int rc = tune_shapes(I->stream, K.has_line, run, S);
     if (rc) return rc;
     // the timed launches wrote the fields: zero them as creation leaves them
     const size_t fbytes = (size_t) I->geo.plane * I->geo.n2 * sizeof(double);
@@ -1598,23 +1632,22 @@ int tune_batch(const std::vector<cf_instance*>& v, cudaStream_t st, LaunchShape&
         v[m]->substep = sub[m];
     }
     if (rc) return rc;
-    std::vector<BatchRec<SolveBatch>> back4;
+    std::vector<BatchRec<SolveBatch>> line;
     std::vector<BatchRec<PoissonArgs>> pois;
     std::vector<BatchRec<ProjArgs>> proj;
     for (const BatchStage& S : K.stages) {
-        if (S.kind == ST_BACK4) back4 = S.back4;
+        if (S.kind == ST_LINE) line = S.line;
         if (S.kind == ST_PSOLVE) pois = S.poisson;
         if (S.kind == ST_PROJECT) proj = S.project;
     }
-    if (back4.size() != v.size() || pois.size() != v.size() || proj.size() != v.size()) return CF_OK;
-    // scratch: four fields and two row-sum blocks per member
+    if (line.size() != v.size() || pois.size() != v.size() || proj.size() != v.size()) return CF_OK;
+    // scratch: four fields and two blocks of column sums per member
     size_t need = 0;
     std::vector<size_t> off(v.size());
     for (size_t m = 0; m < v.size(); m++) {
         const Geo& G = v[m]->geo;
-        const size_t nw = (size_t) ((G.plane + SOLVE_THREADS_MAX - 1) / SOLVE_THREADS_MAX) * (SOLVE_THREADS_MAX / 32);
         off[m] = need;
-        need += 4 * (size_t) G.plane * G.n2 + 2 * nw * G.n2;
+        need += 4 * (size_t) G.plane * G.n2 + 2 * LINE_STATS * (size_t) line_groups(G);
     }
     size_t free_b = 0, total_b = 0;
     CF_CUDA(cudaMemGetInfo(&free_b, &total_b));
@@ -1625,10 +1658,9 @@ int tune_batch(const std::vector<cf_instance*>& v, cudaStream_t st, LaunchShape&
         const Geo& G = v[m]->geo;
         const size_t fsz = (size_t) G.plane * G.n2;
         double* base = scr + off[m];
-        const size_t nw = (size_t) ((G.plane + SOLVE_THREADS_MAX - 1) / SOLVE_THREADS_MAX) * (SOLVE_THREADS_MAX / 32);
-        for (int q = 0; q < 4; q++) back4[m].A.a[q].x = base + q * fsz;
-        back4[m].A.a[0].partial = back4[m].A.a[0].partial ? base + 4 * fsz : nullptr;
-        back4[m].A.a[2].partial = back4[m].A.a[2].partial ? base + 4 * fsz + nw * G.n2 : nullptr;
+        for (int q = 0; q < 4; q++) line[m].A.a[q].x = base + q * fsz;
+        line[m].A.a[0].partial = base + 4 * fsz;
+        line[m].A.a[2].partial = base + 4 * fsz + LINE_STATS * line_groups(G);
         proj[m].A.u = base;
         proj[m].A.v = base + fsz;
         proj[m].A.w = base + 2 * fsz;
@@ -1648,9 +1680,9 @@ int tune_batch(const std::vector<cf_instance*>& v, cudaStream_t st, LaunchShape&
         auto order = [](const auto& r) { return r.G.order; };
         auto none = [](const auto&) { return 0; };
         if (kind == 0) {
-            auto recs = back4;
-            for (auto& r : recs) { r.G.shape = sh; dim3 g = grid_back4(r.G); r.gx = g.x; r.gy = g.y; r.gz = g.z; }
-            add_groups(P, BK_BACK4, recs, order, none, back4_block(recs));
+            auto recs = line;
+            for (auto& r : recs) { r.G.shape = sh; dim3 g = grid_line(r.G); r.gx = g.x; r.gy = g.y; r.gz = g.z; }
+            add_groups(P, BK_LINE, recs, order, none, line_block(recs));
         } else if (kind == 1) {
             auto recs = pois;
             for (auto& r : recs) { r.G.shape = sh; dim3 g = grid_poisson(r.G); r.gx = g.x; r.gy = g.y; r.gz = g.z; }
@@ -1707,7 +1739,7 @@ int cf_destroy(cf_instance* I)
     if (I->graph) cudaGraphDestroy(I->graph);
     // fbuf[0] and gbuf[0] are the bases of the two four-field blocks
     void* bufs[] = {I->u, I->v, I->w, I->c, I->p, I->fbuf[0], I->gbuf[0], I->spec, I->scratch, I->partial,
-                    I->partial_c, I->avg, I->avg_c, I->dscal, I->dcount, I->dlog, I->staging, I->coef, I->twx,
+                    I->partial_c, I->csum, I->avg, I->avg_c, I->dscal, I->dcount, I->dlog, I->staging, I->coef, I->twx,
                     I->twy};
     for (void* b : bufs)
         if (b) cudaFree(b);
@@ -1733,6 +1765,9 @@ static int create_impl(const cf_config* cfg, void* stream, cf_instance* I)
     G.nkx = C.nx / 2 + 1;
     G.plane = (long long) C.nx * C.ny;
     G.splane = (long long) G.nkx * C.ny;
+    int sms = 0;
+    CF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, I->device));
+    G.partitioned = line_partitioned(C.scheme == CF_SCHEME_CHANNEL, G, sms);
     G.dx = I->m.dx;
     G.dy = I->m.dy;
     G.dxdy = I->m.dx * I->m.dy;
@@ -1765,10 +1800,13 @@ static int create_impl(const cf_config* cfg, void* stream, cf_instance* I)
     size_t nscratch = (size_t) nscr * G.splane * G.n2;
     if (helm_fused(I)) nscratch = std::max(nscratch, 4 * helm_scratch_stride(I));   // one per field
     CF_CUDA(cudaMalloc(&I->scratch, nscratch * sizeof(double)));
-    // per-warp partial sums of k_back4, for its largest block size
-    const long long nwarps = ((G.plane + SOLVE_THREADS_MAX - 1) / SOLVE_THREADS_MAX) * (SOLVE_THREADS_MAX / 32);
-    CF_CUDA(cudaMalloc(&I->partial, (size_t) nwarps * G.n2 * sizeof(double)));
-    CF_CUDA(cudaMalloc(&I->partial_c, (size_t) nwarps * G.n2 * sizeof(double)));
+    // column sums of k_line and the controls' sums
+    const size_t nsum = (size_t) LINE_STATS * line_groups(G);
+    CF_CUDA(cudaMalloc(&I->partial, nsum * sizeof(double)));
+    CF_CUDA(cudaMalloc(&I->partial_c, nsum * sizeof(double)));
+    CF_CUDA(cudaMalloc(&I->csum, (2 * LINE_STATS + 1) * sizeof(double)));
+    CF_CUDA(cudaMemsetAsync(I->csum, 0, (2 * LINE_STATS + 1) * sizeof(double), I->stream));
+    I->rhs_rows = rhs_chunk(G, std::max(sms, 1), C.scheme != CF_SCHEME_CHANNEL && !G.partitioned);
     CF_CUDA(cudaMalloc(&I->avg, (size_t) G.n2 * sizeof(double)));
     CF_CUDA(cudaMalloc(&I->avg_c, (size_t) G.n2 * sizeof(double)));
     CF_CUDA(cudaMalloc(&I->dscal, 8 * sizeof(double)));
@@ -2451,8 +2489,8 @@ unsigned long long cf_instance_bytes(const cf_config* c)
         scr = std::max(scr, 4 * per) + 65536;
     }
     b += scr;
-    const unsigned long long nwarps = (plane + SOLVE_THREADS_MAX - 1) / SOLVE_THREADS_MAX * (SOLVE_THREADS_MAX / 32);
-    b += 2 * nwarps * n2 * 8 + 2 * n2 * 8 + 64 + 8;                            // row sums, averages, scalars
+    const unsigned long long nsum = (plane + 15) / 16 * LINE_STATS;
+    b += 2 * nsum * 8 + 2 * n2 * 8 + (2 * LINE_STATS + 1) * 8 + 64 + 8;        // column sums, averages, scalars
     b += 3ull * 4096 * LOG_COLS * 8;                                           // log ring
     b += (unsigned long long) (c->nx + c->ny) * 16;                            // twiddles
     b += n2 * 8 * 512 + (unsigned long long) (c->nx + c->ny) * 8;              // coefficient tables (bound)
@@ -2479,16 +2517,15 @@ int cf_pressure_fused(const cf_instance* I)
 int cf_launches_per_substep(const cf_instance* I)
 {
     // pressure: div+fftx (two launches for power-of-two nx), ffty, poisson,
-    // ffty, fftx_c2r, project.  chanfast: ghosts, rhs + forward sweeps, the
-    // four back substitutions, 2 x (row average + mass control).  channel
-    // (power-of-two nx only): ghosts, rhs + Helmholtz right-hand sides, fftx,
-    // ffty, four spectral solves, ffty, fftx_c2r, apply_bc, 2 x mass control.
-    // With power-of-two ny the y transforms and the Poisson solve are one
-    // launch (two fewer).
+    // ffty, fftx_c2r, project.  chanfast: ghosts, rhs, the line solves, the
+    // two controls in one launch.  channel (power-of-two nx only): ghosts,
+    // rhs + Helmholtz right-hand sides, fftx, ffty, four spectral solves, ffty,
+    // fftx_c2r, apply_bc, 2 x mass control.  Where the y transforms and the
+    // Poisson solve are one launch, two fewer.
     if (!I) return CF_EINVAL;
     const int pressure = (fftx_batched_supported(I->cfg.nx) ? 7 : 6) - (I->fuse_pressure && poisson_fft_supported(I->geo) ? 2 : 0);
     // the channel scheme's y transforms and four spectral solves: 6 launches, or 1 fused
-    return (I->cfg.scheme == CF_SCHEME_CHANNEL ? (helm_fused(I) ? 8 : 13) : 7) + pressure;
+    return (I->cfg.scheme == CF_SCHEME_CHANNEL ? (helm_fused(I) ? 8 : 13) : 4) + pressure;
 }
 
 }  // extern "C"

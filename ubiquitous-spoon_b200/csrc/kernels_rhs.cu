@@ -15,12 +15,10 @@
 #include "wall.cuh"
 #include "batch.cuh"
 
+#include <algorithm>
 #include <type_traits>
 
 namespace cf {
-
-__device__ __forceinline__ int wrapi(int a, int n) { return a < 0 ? a + n : (a >= n ? a - n : a); }
-
 
 // ------------------------------------------------------------------ ghosts
 
@@ -87,8 +85,8 @@ __global__ void k_ghosts_batch(const BatchRec<GhostArgs>* r, int n)
 
 // --------------------------------------------------------------------- RHS
 //
-// One block owns an 8 (x) by 32 (y) column tile and marches up all interior
-// rows.  The 7 k-planes a row needs (k-3..k+3) of u, v, w, c, with a
+// One block owns an 8 (x) by 32 (y) column tile and marches up its rows.
+// The 7 k-planes a row needs (k-3..k+3) of u, v, w, c, with a
 // periodic halo of 3 rows in x and 4 columns in y, sit in a ring of 8
 // shared-memory slots; the next plane streams in with cp.async while the
 // current row is computed.  Every
@@ -96,18 +94,22 @@ __global__ void k_ghosts_batch(const BatchRec<GhostArgs>* r, int n)
 // are multiplications by their reciprocals (host tables), so results agree
 // with the reference to rounding, not bit for bit.
 //
-// After a row's four right-hand sides the same thread runs that row of the
-// forward sweeps of the four implicit solves (chanfast.c:459-482 with the
-// forward half of tridag/heptdag): the old field window x_{k-H..k+H} is in
-// the ring, f was just computed, g is read and overwritten by s.  The back
-// substitution follows in k_back4 (kernels_solve.cu).
-//
-// IMPL3D (the fully implicit scheme of channel.c): f has no x-y diffusion
-// (channel.c:419-438), and in place of the sweep row each thread forms the
-// Helmholtz right-hand side h = x + nuadt (Lxy + Lz) x + gamdt f + zetdt g
-// - hbc (channel.c:455-467, 531-543, 560-572, 636-648) of its point, which
-// overwrites g; A.nu and A.kappa then carry nuadt and nuadt / prandtl.  The
-// spectral solves follow (kernels_pressure.cu).
+// After a row's four right-hand sides the same thread forms the right-hand
+// sides h of the four implicit solves (chanfast.c:459-480): the old field
+// window x_{k-H..k+H} is in the ring, f was just computed, g is read and
+// overwritten.
+// MODE RHS_SWEEP: it also runs that row of the solves' forward sweeps (the
+//   forward half of tridag/heptdag), leaving s; a block marches up all
+//   interior rows, and the back sweep follows in k_line (kernels_solve.cu).
+// MODE RHS_H: h itself is left; no row depends on the rows below it beyond the
+//   carried fluxes, so a block takes A.chunk rows of its tile (rhs_chunk),
+//   and both sweeps follow in k_line.
+// MODE RHS_CHANNEL (the fully implicit scheme of channel.c), rows as RHS_H: f
+//   has no x-y diffusion (channel.c:419-438) and h = x + nuadt (Lxy + Lz) x +
+//   gamdt f + zetdt g - hbc (channel.c:455-467, 531-543, 560-572, 636-648);
+//   A.nu and A.kappa then carry nuadt and nuadt / prandtl.  The spectral
+//   solves follow (kernels_pressure.cu).
+enum RhsMode { RHS_SWEEP, RHS_H, RHS_CHANNEL };
 
 constexpr int RT_I = 8, RT_J = 32;
 constexpr int RT_THREADS = RT_I * RT_J;
@@ -202,7 +204,7 @@ __device__ __forceinline__ void cp_async16(double* dst, const double* src)   // 
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
-template <int ORDER, bool IMPL3D>
+template <int ORDER, int MODE>
 __device__ __forceinline__ void rhs_body(const Geo& G, const RhsArgs& A, uint3 bid)
 {
     extern __shared__ double sm[];
@@ -211,7 +213,7 @@ __device__ __forceinline__ void rhs_body(const Geo& G, const RhsArgs& A, uint3 b
     const int j0 = bid.x * RT_J, i0 = bid.y * RT_I;
     const int nx = G.nx, ny = G.ny, n2 = G.n2;
     const long long plane = (long long) nx * ny;
-    const int kb = GZ, ke = GZ + G.nz;   // all interior rows: the forward sweeps run in order
+    const int kb = GZ + (int) bid.z * A.chunk, ke = min(kb + A.chunk, GZ + G.nz);   // RHS_SWEEP: all interior rows, in order
 
     // This thread's points (even ny: pairs of points) of a haloed plane,
     // the same in every plane: their offsets within a field plane, computed
@@ -384,7 +386,8 @@ __device__ __forceinline__ void rhs_body(const Geo& G, const RhsArgs& A, uint3 b
         double sk = r[2 * H + 3] + r[2 * H + 1] * fk + r[2 * H + 2] * gk;
 #pragma unroll
         for (int q = 0; q < 2 * H + 1; q++) sk += r[q] * X(q - H);
-        if (IMPL3D) return sk + lk;   // h of this point (channel_rows: no elimination)
+        if (MODE == RHS_CHANNEL) return sk + lk;
+        if (MODE == RHS_H) return sk;
         if (ORDER == 4) sk -= r[2 * H + 5] * s2 + r[2 * H + 6] * s3;
         sk -= r[2 * H + 4] * s1;   // the previous row's s enters last
         s3 = s2; s2 = s1; s1 = sk;
@@ -538,12 +541,12 @@ __device__ __forceinline__ void rhs_body(const Geo& G, const RhsArgs& A, uint3 b
             if (do_w) lw = lap4(W, A.nu);
             lc = lap4(C, A.kappa);
         }
-        if (!IMPL3D) {
+        if (MODE != RHS_CHANNEL) {
             fu += lu;
             fv += lv;
             fw += lw;
         }
-        fc = IMPL3D ? 0.0 : lc;
+        fc = MODE == RHS_CHANNEL ? 0.0 : lc;
 
         {   // flux_quick + advect_scalar (scalar.c:79-162), order independent
             const double c0 = C(0, 0, 0);
@@ -617,10 +620,10 @@ __device__ __forceinline__ void rhs_body(const Geo& G, const RhsArgs& A, uint3 b
     }
 }
 
-template <int ORDER, bool IMPL3D>
+template <int ORDER, int MODE>
 __global__ void __launch_bounds__(RT_THREADS, RhsTile<ORDER>::BLOCKS) k_rhs(Geo G, RhsArgs A)
 {
-    rhs_body<ORDER, IMPL3D>(G, A, blockIdx);
+    rhs_body<ORDER, MODE>(G, A, blockIdx);
 }
 
 template <int ORDER>
@@ -628,7 +631,7 @@ __global__ void __launch_bounds__(RT_THREADS, RhsTile<ORDER>::BLOCKS) k_rhs_batc
 {
     uint3 b;
     const BatchRec<RhsArgs>& R = batch_locate(r, n, b);
-    rhs_body<ORDER, false>(R.G, R.A, b);
+    rhs_body<ORDER, RHS_SWEEP>(R.G, R.A, b);
 }
 
 // ------------------------------------------------------------- launchers
@@ -650,7 +653,37 @@ void launch_ghosts(const Geo& G, const GhostArgs& A, cudaStream_t st, bool extra
     }
 }
 
-dim3 grid_rhs(const Geo& G) { return dim3((G.ny + RT_J - 1) / RT_J, (G.nx + RT_I - 1) / RT_I, 1); }
+dim3 grid_rhs(const Geo& G, int chunk)
+{
+    return dim3((G.ny + RT_J - 1) / RT_J, (G.nx + RT_I - 1) / RT_I, (G.nz + chunk - 1) / chunk);
+}
+
+long long rhs_tiles(const Geo& G) { return (long long) ((G.ny + RT_J - 1) / RT_J) * ((G.nx + RT_I - 1) / RT_I); }
+
+// Rows per k_rhs block of an instance that runs alone.  One block fills an
+// SM, so the time is the number of waves times a block's rows plus its
+// start (the ring's first planes and the primed fluxes, about RHS_START
+// rows); the chunk count with the least of it is taken.  Whole columns with
+// the forward sweep in the kernel (sweep), and where the tiles alone give
+// three quarters of the SMs a block (as line_partitioned).
+int rhs_chunk(const Geo& G, int sms, bool sweep)
+{
+    constexpr int RHS_START = 4;
+    const long long tiles = rhs_tiles(G);
+    if (sweep || 4 * tiles > 3 * sms) return G.nz;
+    long long best = -1;
+    int chunk = G.nz;
+    for (int c = 1; c <= std::max(1, G.nz / RHS_MIN_ROWS); c++) {
+        const int rows = (G.nz + c - 1) / c;
+        const long long n = (G.nz + rows - 1) / rows, waves = (tiles * n + sms - 1) / sms;
+        const long long cost = waves * (rows + RHS_START);
+        if (best < 0 || cost < best) {
+            best = cost;
+            chunk = rows;
+        }
+    }
+    return chunk;
+}
 
 void launch_ghosts_batch(const BatchLaunch& L, int order, cudaStream_t st)
 {
@@ -659,36 +692,40 @@ void launch_ghosts_batch(const BatchLaunch& L, int order, cudaStream_t st)
     else k_ghosts_batch<4, true><<<L.blocks, GHOST_THREADS, 0, st>>>(r, L.n);
 }
 
+// (whole columns in a batch: line_partitioned)
 void launch_rhs_batch(const BatchLaunch& L, int order, cudaStream_t st)
 {
     auto r = static_cast<const BatchRec<RhsArgs>*>(L.recs);
-    dim3 blk(RT_J, RT_I, 1);
+    const dim3 blk(RT_J, RT_I, 1);
     if (order == 2) k_rhs_batch<2><<<L.blocks, blk, rhs_smem_bytes<2>(), st>>>(r, L.n);
     else k_rhs_batch<4><<<L.blocks, blk, rhs_smem_bytes<4>(), st>>>(r, L.n);
 }
 
 void launch_rhs(const Geo& G, const RhsArgs& A, bool implicit3d, cudaStream_t st)
 {
-    dim3 blk(RT_J, RT_I, 1);
-    dim3 grd = grid_rhs(G);
-    if (implicit3d) {
-        if (G.order == 2) k_rhs<2, true><<<grd, blk, rhs_smem_bytes<2>(), st>>>(G, A);
-        else k_rhs<4, true><<<grd, blk, rhs_smem_bytes<4>(), st>>>(G, A);
-    } else {
-        if (G.order == 2) k_rhs<2, false><<<grd, blk, rhs_smem_bytes<2>(), st>>>(G, A);
-        else k_rhs<4, false><<<grd, blk, rhs_smem_bytes<4>(), st>>>(G, A);
-    }
+    const dim3 blk(RT_J, RT_I, 1), grd = grid_rhs(G, A.chunk);
+    const int mode = implicit3d ? RHS_CHANNEL : G.partitioned ? RHS_H : RHS_SWEEP;
+#define CASE_(o_, m_) if (G.order == o_ && mode == m_) k_rhs<o_, m_><<<grd, blk, rhs_smem_bytes<o_>(), st>>>(G, A);
+    CASE_(2, RHS_SWEEP) CASE_(2, RHS_H) CASE_(2, RHS_CHANNEL)
+    CASE_(4, RHS_SWEEP) CASE_(4, RHS_H) CASE_(4, RHS_CHANNEL)
+#undef CASE_
 }
 
 cudaError_t rhs_set_smem_limits()
 {
     const int v2 = (int) rhs_smem_bytes<2>(), v4 = (int) rhs_smem_bytes<4>();
-    cudaError_t e = cudaFuncSetAttribute(k_rhs<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, v2);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_rhs<4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, v4);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_rhs<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, v2);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_rhs<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, v4);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_rhs_batch<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, v2);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_rhs_batch<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, v4);
+    cudaError_t e = cudaSuccess;
+    auto set = [&](const void* f, int v) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
+    };
+    set((const void*) k_rhs<2, RHS_SWEEP>, v2);
+    set((const void*) k_rhs<2, RHS_H>, v2);
+    set((const void*) k_rhs<2, RHS_CHANNEL>, v2);
+    set((const void*) k_rhs<4, RHS_SWEEP>, v4);
+    set((const void*) k_rhs<4, RHS_H>, v4);
+    set((const void*) k_rhs<4, RHS_CHANNEL>, v4);
+    set((const void*) k_rhs_batch<2>, v2);
+    set((const void*) k_rhs_batch<4>, v4);
     return e;
 }
 
