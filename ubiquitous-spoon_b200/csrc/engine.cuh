@@ -219,7 +219,8 @@ struct PoissonArgs {
 
 // k_poisson block: one thread per (kx, +-ky) column pair, LaunchShape::pois_threads per block
 constexpr int POIS_PF = 8;         // forward rows in flight per thread (both columns)
-constexpr int POIS_PB = 2;         // back-substitution rows loaded ahead (registers)
+constexpr int POIS_PB = 4;         // back-substitution rows loaded ahead (registers)
+constexpr int POIS_PB2 = 6;        // at order 2
 inline size_t pois_smem_bytes(int threads) { return (size_t) POIS_PF * 2 * threads * 16; }
 
 // k_poisson_fft: forward y transform + Poisson solve (with the wall ghost

@@ -573,16 +573,18 @@ struct PairRows {
         default: return A.dvol[k];
         }
     }
-    // Coefficients of interior row i (k = GZ + i).
-    __device__ __forceinline__ void coef(int i, double* cf) const
+    // Table values of row k = GZ + i for coef_from, and the cell volume, st[9].
+    template <int ORDER>
+    __device__ __forceinline__ void load(int i, double* st) const
     {
-        const int k = GZ + i;
-        double st[9] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, A.dpart[k], A.cx[k], A.cy[k]};
-        if (bq(i) < 0) {   // closure rows take their band from red
-            st[0] = A.a[k]; st[1] = A.b[k]; st[2] = A.c[k];
-            st[3] = A.e[k]; st[4] = A.f[k]; st[5] = A.g[k];
+        const int k = GZ + min(i, n - 1);
+        st[6] = __ldg(A.dpart + k); st[7] = __ldg(A.cx + k); st[8] = __ldg(A.cy + k); st[9] = __ldg(A.dvol + k);
+        st[0] = __ldg(A.a + k); st[2] = __ldg(A.c + k);
+        if (ORDER == 4) {
+            st[1] = __ldg(A.b + k); st[3] = __ldg(A.e + k); st[4] = __ldg(A.f + k); st[5] = __ldg(A.g + k);
+        } else {
+            st[1] = st[3] = st[4] = st[5] = 0.0;
         }
-        coef_from(i, st, cf);
     }
 };
 
@@ -635,6 +637,13 @@ __device__ __forceinline__ double2 hept_back(double2 sv, double p, double q, dou
 // eliminates both (Re and Im of each), storing the multipliers once.  ky = 0
 // and, for even ny, ky = ny/2 pair with themselves (solved twice, stored
 // identically).
+//
+// Bound: latency of the two sweeps (few columns) or the spectrum's and the
+// multipliers' traffic (many).  Both sweeps read ahead, 8 rows forward and 4
+// (order 2: 6) back, and the band tables one row; at order 2, which read each
+// row when it came to it, 107 -> 52 us at 192 x 192 x 128 and 47 -> 28 us at
+// 64 x 64 x 64; at order 4, which read back two rows ahead, 67 -> 56 us at
+// 128 x 128 x 96.
 template <int ORDER, bool FILL>
 __device__ __forceinline__ void band_column(const Geo& G, const PoissonArgs& A, uint3 bid)
 {
@@ -655,55 +664,97 @@ __device__ __forceinline__ void band_column(const Geo& G, const PoissonArgs& A, 
     auto SB = [&](int k) -> double2& { return sp[(long long) k * ncol + colB]; };
     auto scal = [](double2 v, double f) { return make_double2(v.x * f, v.y * f); };
     const PairRows rows{A, lamx, lamy, var, n};
-    auto coef = [&](int i, double* cf) { rows.coef(i, cf); };
     auto at = [&](double* base, int k) -> double& { return base[(long long) k * npair + pair]; };
+
+    // In the forward sweep each thread keeps the spectrum values of the next
+    // POIS_PF rows of both columns in flight as cp.async copies into its own
+    // slots of a shared-memory ring (none of those rows has been rewritten
+    // yet), and the band tables of the next row in registers.
+    extern __shared__ double2 pring[];
+    const int t = threadIdx.x;
+    const int nt = blockDim.x;
+    auto fslot = [&](int i, int c) { return pring + ((i % POIS_PF) * 2 + c) * nt + t; };
+    auto ffetch = [&](int i) {
+        if (i < n) {
+            cp_async16_ordered(fslot(i, 0), &SA(GZ + i));
+            cp_async16_ordered(fslot(i, 1), &SB(GZ + i));
+        }
+        cp_async_commit_ordered();
+    };
+    for (int i = 0; i < POIS_PF; i++) ffetch(i);
+    double cf[7], st[10], sn[10];
+    rows.load<ORDER>(0, sn);
+    // row i: its right-hand sides scaled by the cell volume, its band in cf
+    auto next_row = [&](int i, double2& hA, double2& hB) {
+#pragma unroll
+        for (int q = 0; q < 10; q++) st[q] = sn[q];
+        rows.load<ORDER>(i + 1, sn);
+        cp_async_wait_ordered<POIS_PF - 1>();
+        hA = scal(*fslot(i, 0), st[9]);
+        hB = scal(*fslot(i, 1), st[9]);
+        ffetch(i + POIS_PF);
+        rows.coef_from(i, st, cf);
+    };
 
     if (ORDER == 2) {
         // tridag.c:4-26; the diagonal is cf[3], the off-diagonals cf[0], cf[2]
         double* gam = A.scratch;
-        double cfv[7];
-        coef(0, cfv);
-        double ibet = 1.0 / cfv[3];
-        const double dv0 = A.dvol[GZ];
-        const double2 r0A = SA(GZ), r0B = SB(GZ);
-        double2 uA = make_double2(r0A.x * dv0 * ibet, r0A.y * dv0 * ibet);
-        double2 uB = make_double2(r0B.x * dv0 * ibet, r0B.y * dv0 * ibet);
-        SA(GZ) = uA;
-        SB(GZ) = uB;
-        double cprev = cfv[2];
-        for (int i = 1; i < n; i++) {
+        double2 uA = make_double2(0.0, 0.0), uB = uA;
+        double ibet = 0.0, cprev = 0.0;
+        for (int i = 0; i < n; i++) {
             const int k = GZ + i;
-            coef(i, cfv);
-            double gm = cprev * ibet;
-            ibet = 1.0 / (cfv[3] - cfv[0] * gm);
+            double2 hA, hB;
+            next_row(i, hA, hB);
+            // (row 0: no history, ibet = cprev = 0)
+            const double gm = cprev * ibet;
+            ibet = 1.0 / (i ? cf[3] - cf[0] * gm : cf[3]);
             at(gam, k) = gm;
-            const double dv = A.dvol[k];
-            const double2 rA = SA(k), rB = SB(k);
-            uA = make_double2((rA.x * dv - cfv[0] * uA.x) * ibet, (rA.y * dv - cfv[0] * uA.y) * ibet);
-            uB = make_double2((rB.x * dv - cfv[0] * uB.x) * ibet, (rB.y * dv - cfv[0] * uB.y) * ibet);
+            uA = make_double2((i ? hA.x - cf[0] * uA.x : hA.x) * ibet, (i ? hA.y - cf[0] * uA.y : hA.y) * ibet);
+            uB = make_double2((i ? hB.x - cf[0] * uB.x : hB.x) * ibet, (i ? hB.y - cf[0] * uB.y : hB.y) * ibet);
             SA(k) = uA;
             SB(k) = uB;
-            cprev = cfv[2];
+            cprev = cf[2];
         }
+        cp_async_wait_ordered<0>();
+        // back sweep; POIS_PB2 rows are loaded ahead (plain loads: this thread stored them)
         double2 nA = uA, nB = uB;
         const double2 topA = uA, topB = uB;
         double2 b0A = uA, b0B = uB;
         if (stats) A.avg[GZ + n - 1] = uA.x;
-        for (int i = n - 2; i >= 0; i--) {
-            const int k = GZ + i;
-            const double gm = at(gam, k + 1);
-            double2 tA = SA(k), tB = SB(k);
-            tA.x -= gm * nA.x;
-            tA.y -= gm * nA.y;
-            tB.x -= gm * nB.x;
-            tB.y -= gm * nB.y;
-            SA(k) = tA;
-            SB(k) = tB;
-            nA = tA;
-            nB = tB;
-            if (stats) A.avg[k] = tA.x;
-            if (i == 0) { b0A = tA; b0B = tB; }
+        double2 lA[POIS_PB2], lB[POIS_PB2];
+        double lg[POIS_PB2];
+        auto bload = [&](int i, int u) {
+            if (i >= 0) {
+                lA[u] = SA(GZ + i);
+                lB[u] = SB(GZ + i);
+                lg[u] = at(gam, GZ + i + 1);
+            }
+        };
+#pragma unroll
+        for (int u = 0; u < POIS_PB2; u++) bload(n - 2 - u, u);
+        for (int i0 = n - 2; i0 >= 0; i0 -= POIS_PB2) {
+#pragma unroll
+            for (int u = 0; u < POIS_PB2; u++) {
+                const int i = i0 - u;
+                if (i >= 0) {
+                    const int k = GZ + i;
+                    double2 tA = lA[u], tB = lB[u];
+                    const double gm = lg[u];
+                    bload(i - POIS_PB2, u);
+                    tA.x -= gm * nA.x;
+                    tA.y -= gm * nA.y;
+                    tB.x -= gm * nB.x;
+                    tB.y -= gm * nB.y;
+                    SA(k) = tA;
+                    SB(k) = tB;
+                    nA = tA;
+                    nB = tB;
+                    if (stats) A.avg[k] = tA.x;
+                }
+            }
         }
+        b0A = nA;
+        b0B = nB;
         if (FILL) {
             auto fill = [&](auto S, double2 b0, double2 top) {
                 double g1, g2, g3, h1;
@@ -728,36 +779,15 @@ __device__ __forceinline__ void band_column(const Geo& G, const PoissonArgs& A, 
         return;
     }
 
-    // heptdag.c:5-61 with per-pair pivots (HeptSweep); p, q, r spill to
-    // scratch.  In the forward sweep each thread keeps the spectrum values of the next
-    // POIS_PF rows of both columns in flight as cp.async copies into its own
-    // slots of a shared-memory ring; none of those rows has been rewritten yet.
+    // heptdag.c:5-61 with per-pair pivots (HeptSweep); p, q, r spill to scratch
     double* Pp = A.scratch;
     double* Qp = A.scratch + (long long) n2 * npair;
     double* Rp = A.scratch + 2 * (long long) n2 * npair;
-    extern __shared__ double2 pring[];
-    const int t = threadIdx.x;
-    const int nt = blockDim.x;
-    auto fslot = [&](int i, int c) { return pring + ((i % POIS_PF) * 2 + c) * nt + t; };
-    auto ffetch = [&](int i) {
-        if (i < n) {
-            cp_async16_ordered(fslot(i, 0), &SA(GZ + i));
-            cp_async16_ordered(fslot(i, 1), &SB(GZ + i));
-        }
-        cp_async_commit_ordered();
-    };
-    for (int i = 0; i < POIS_PF; i++) ffetch(i);
     HeptSweep H;
-    double cf[7];
     for (int i = 0; i < n; i++) {
         const int k = GZ + i;
-        cp_async_wait_ordered<POIS_PF - 1>();
-        double2 hA = *fslot(i, 0), hB = *fslot(i, 1);
-        ffetch(i + POIS_PF);
-        coef(i, cf);
-        const double dv = A.dvol[k];
-        hA = scal(hA, dv);
-        hB = scal(hB, dv);
+        double2 hA, hB;
+        next_row(i, hA, hB);
         double p, q, r;
         double2 svA, svB;
         H.step(cf, hA, hB, p, q, r, svA, svB);
@@ -2093,7 +2123,7 @@ void launch_poisson(const Geo& G, const PoissonArgs& A, cudaStream_t st)
 {
     unsigned nb = grid_poisson(G).x;
     const int nt = G.shape.pois_threads;
-    if (G.order == 2) k_poisson<2><<<nb, nt, 0, st>>>(G, A);
+    if (G.order == 2) k_poisson<2><<<nb, nt, pois_smem_bytes(nt), st>>>(G, A);
     else k_poisson<4><<<nb, nt, pois_smem_bytes(nt), st>>>(G, A);
 }
 
@@ -2101,7 +2131,7 @@ void launch_helmholtz_spectral(const Geo& G, const PoissonArgs& A, cudaStream_t 
 {
     unsigned nb = grid_poisson(G).x;
     const int nt = G.shape.pois_threads;
-    if (G.order == 2) k_helmholtz_spectral<2><<<nb, nt, 0, st>>>(G, A);
+    if (G.order == 2) k_helmholtz_spectral<2><<<nb, nt, pois_smem_bytes(nt), st>>>(G, A);
     else k_helmholtz_spectral<4><<<nb, nt, pois_smem_bytes(nt), st>>>(G, A);
 }
 
@@ -2214,7 +2244,7 @@ void launch_ffty_batch(const BatchLaunch& L, int ny, cudaStream_t st)
 
 void launch_poisson_batch(const BatchLaunch& L, int order, cudaStream_t st)
 {
-    if (order == 2) k_poisson_batch<2><<<L.blocks, L.block, 0, st>>>(recs_of<PoissonArgs>(L), L.n);
+    if (order == 2) k_poisson_batch<2><<<L.blocks, L.block, pois_smem_bytes(L.block.x), st>>>(recs_of<PoissonArgs>(L), L.n);
     else k_poisson_batch<4><<<L.blocks, L.block, pois_smem_bytes(L.block.x), st>>>(recs_of<PoissonArgs>(L), L.n);
 }
 
