@@ -165,7 +165,8 @@ __device__ void fft_run(const FftCtx& F, const FftPlan& plan)
     }
 }
 
-constexpr int FFT_L = 8;        // lines per block (x transforms: 8 consecutive j)
+constexpr int FFT_L = 8;        // transforms per block
+constexpr int FFT_J = 16;       // columns of an x-transform block, two per transform
 constexpr int FFT_THREADS = 256;
 constexpr int FFT_MAXC = 16;    // N * L / threads for N <= 512
 
@@ -302,21 +303,30 @@ size_t fft_generic_smem(int n, bool line_major)
 // --------------------------------------------------------- divergence + x FFT
 
 
+// Two real lines, columns j and j + 1, ride through one complex transform as
+// its real and imaginary part: Z = A + i B with A, B Hermitian, so that
+// A[k] = (Z[k] + conj Z[N-k]) / 2, B[k] = (Z[k] - conj Z[N-k]) / 2i.  A block's
+// FFT_L transforms take FFT_J = 16 columns, a 128-byte row segment.  One real
+// line per transform did twice the work and read half a segment: the inverse at
+// 192 x 192 x 128 44 -> 26 us, at 90 x 75 x 53 (runtime plan) 27 -> 17 us, the
+// divergence with its transform 95 -> 83 and 33 -> 23 us.
+//
 // N: the transform size when it is fixed at compile time, 0 for the runtime plan
 template <int ORDER, int N>
 __device__ __forceinline__ void k_div_fftx_body(const Geo& G, const DivArgs& A, uint3 bid)
 {
     extern __shared__ double2 sbuf[];
+    double* const sreal = reinterpret_cast<double*>(sbuf);   // [pos][column]
     const int k = GZ + A.kshift + bid.y;
-    const int j0 = bid.x * FFT_L;
+    const int j0 = bid.x * FFT_J;
     const int nx = N ? N : G.nx, ny = G.ny, n2 = G.n2;
     const double dx = G.dx, dy = G.dy, dzk = G.dz[k];
     const double uc = A.mu ? A.gu[k] * (*A.mu) : 0.0;   // chanfast.c:516-519
     const bool corr = A.mu != nullptr;
     auto I = [&](int kk, int i, int j) { return ((long long) kk * nx + i) * ny + j; };
     const int kb = GZ - 1, kt = n2 - GZ - 1;
-    for (int idx = threadIdx.x; idx < nx * FFT_L; idx += blockDim.x) {
-        int i = idx / FFT_L, jj = idx - i * FFT_L, j = j0 + jj;
+    for (int idx = threadIdx.x; idx < nx * FFT_J; idx += blockDim.x) {
+        int i = idx / FFT_J, jj = idx - i * FFT_J, j = j0 + jj;
         double d = 0.0;
         if (j < ny && A.src) {
             d = __ldg(A.src + I(k, i, j));
@@ -334,21 +344,20 @@ __device__ __forceinline__ void k_div_fftx_body(const Geo& G, const DivArgs& A, 
                   + (A1 * (Wr(k) - Wr(k - 1)) + A2 * (wkp1 - wkm2)) / dzk;
             }
         }
-        sbuf[i * FFT_L + jj] = make_double2(d, 0.0);
+        sreal[idx] = d;
     }
     __syncthreads();
     FftCtx F{sbuf, nx, FFT_L, false, -1, A.px.tw, A.c8};
     if constexpr (N > 0) fft_static<N, false>(sbuf, F);
     else fft_run<FFT_MAXC>(F, A.px);
     const int nkx = G.nkx;
-    const double scale = 1.0 / (double) nx;
-    for (int idx = threadIdx.x; idx < nkx * FFT_L; idx += blockDim.x) {
-        int kx = idx / FFT_L, jj = idx - kx * FFT_L, j = j0 + jj;
+    const double scale = 0.5 / (double) nx;
+    for (int idx = threadIdx.x; idx < nkx * FFT_J; idx += blockDim.x) {
+        int kx = idx / FFT_J, jj = idx - kx * FFT_J, j = j0 + jj;
         if (j >= ny) continue;
-        double2 t = sbuf[kx * FFT_L + jj];
-        t.x *= scale;
-        t.y *= scale;
-        A.spec[((long long) k * nkx + kx) * ny + j] = t;
+        const double2 z = sbuf[kx * FFT_L + jj / 2], c = sbuf[(kx ? nx - kx : 0) * FFT_L + jj / 2];
+        const double2 t = jj & 1 ? make_double2(z.y + c.y, c.x - z.x) : make_double2(z.x + c.x, z.y - c.y);
+        A.spec[((long long) k * nkx + kx) * ny + j] = make_double2(t.x * scale, t.y * scale);
     }
 }
 
@@ -419,36 +428,34 @@ __global__ void __launch_bounds__(FFT_THREADS) k_ffty_batch(const BatchRec<FftyA
 // ---------------------------------------------------------- inverse x FFT
 
 
+// Two columns per transform as above: Z[k] = A[k] + i B[k], both completed by
+// Hermitian symmetry; the inverse's real and imaginary part are the lines.
 template <int N>
 __device__ __forceinline__ void k_fftx_c2r_body(const Geo& G, const C2rArgs& A, uint3 bid)
 {
     extern __shared__ double2 sbuf[];
+    const double* const sreal = reinterpret_cast<const double*>(sbuf);
     const int k = A.kfirst + bid.y;
-    const int j0 = bid.x * FFT_L;
+    const int j0 = bid.x * FFT_J;
     const int nx = N ? N : G.nx, ny = G.ny, nkx = G.nkx;
-    const double2* spec = A.spec + bid.z * A.fstride;
-    for (int idx = threadIdx.x; idx < nx * FFT_L; idx += blockDim.x) {
-        int pos = idx / FFT_L, jj = idx - pos * FFT_L, j = j0 + jj;
-        double2 t = make_double2(0.0, 0.0);
-        if (j < ny) {
-            if (pos < nkx) {
-                t = spec[((long long) k * nkx + pos) * ny + j];
-                if (pos == 0 || 2 * pos == nx) t.y = 0.0;
-            } else {
-                t = spec[((long long) k * nkx + (nx - pos)) * ny + j];
-                t.y = -t.y;
-            }
-        }
-        sbuf[pos * FFT_L + jj] = t;
+    const double2* spec = A.spec + bid.z * A.fstride + (long long) k * nkx * ny;
+    for (int idx = threadIdx.x; idx < nkx * FFT_L; idx += blockDim.x) {
+        const int kx = idx / FFT_L, l = idx - kx * FFT_L, j = j0 + 2 * l;
+        double2 a = make_double2(0.0, 0.0), b = a;
+        if (j < ny) a = spec[(long long) kx * ny + j];
+        if (j + 1 < ny) b = spec[(long long) kx * ny + j + 1];
+        if (kx == 0 || 2 * kx == nx) a.y = b.y = 0.0;
+        sbuf[kx * FFT_L + l] = make_double2(a.x - b.y, a.y + b.x);
+        if (kx && 2 * kx != nx) sbuf[(nx - kx) * FFT_L + l] = make_double2(a.x + b.y, b.x - a.y);
     }
     __syncthreads();
     FftCtx F{sbuf, nx, FFT_L, false, +1, A.px.tw, A.c8};
     if constexpr (N > 0) fft_static<N, false>(sbuf, F);
     else fft_run<FFT_MAXC>(F, A.px);
     double* const pz = bid.z == 0 ? A.p[0] : bid.z == 1 ? A.p[1] : bid.z == 2 ? A.p[2] : A.p[3];
-    for (int idx = threadIdx.x; idx < nx * FFT_L; idx += blockDim.x) {
-        int i = idx / FFT_L, jj = idx - i * FFT_L, j = j0 + jj;
-        if (j < ny) pz[((long long) k * nx + i) * ny + j] = sbuf[i * FFT_L + jj].x;
+    for (int idx = threadIdx.x; idx < nx * FFT_J; idx += blockDim.x) {
+        int i = idx / FFT_J, jj = idx - i * FFT_J, j = j0 + jj;
+        if (j < ny) pz[((long long) k * nx + i) * ny + j] = sreal[idx];
     }
 }
 
@@ -1956,7 +1963,7 @@ void launch_div_fftx(const Geo& G, const DivArgs& A, cudaStream_t st)
     case 512: return launch_div_fftx_p2<512>(G, A, st);
     default: break;
     }
-    dim3 grd((G.ny + FFT_L - 1) / FFT_L, G.nz);
+    dim3 grd((G.ny + FFT_J - 1) / FFT_J, G.nz);
     size_t sm = fft_smem_bytes(G.nx);
 #define CASE_(n_) \
     case n_: \
@@ -1985,7 +1992,7 @@ void launch_fft2d_field(const Geo& G, const double* field, double2* spec, const 
         D.c8 = c8;
         D.src = field;
         D.kshift = -GZ;
-        dim3 grd((G.ny + FFT_L - 1) / FFT_L, G.n2);
+        dim3 grd((G.ny + FFT_J - 1) / FFT_J, G.n2);
         const size_t sm = fft_smem_bytes(G.nx);
 #define CASE_(n_) \
     case n_: k_div_fftx<2, n_><<<grd, FFT_THREADS, sm, st>>>(G, D); break;
@@ -2045,7 +2052,7 @@ void launch_fftx_c2r(const Geo& G, const C2rArgs& A, int nrows, cudaStream_t st,
     case 512: return launch_c2r_p2<512>(G, A, nrows, nfields, st);
     default: break;
     }
-    dim3 grd((G.ny + FFT_L - 1) / FFT_L, nrows, nfields);
+    dim3 grd((G.ny + FFT_J - 1) / FFT_J, nrows, nfields);
     const size_t sm = fft_smem_bytes(G.nx);
 #define CASE_(n_) \
     case n_: k_fftx_c2r<n_><<<grd, FFT_THREADS, sm, st>>>(G, A); return;
@@ -2162,7 +2169,7 @@ dim3 grid_r2c(const Geo& G, int nrows, int nfields)
     return dim3((G.ny + L - 1) / L, nrows, nfields);
 }
 
-dim3 grid_div_fftx(const Geo& G) { return dim3((G.ny + FFT_L - 1) / FFT_L, G.nz); }
+dim3 grid_div_fftx(const Geo& G) { return dim3((G.ny + FFT_J - 1) / FFT_J, G.nz); }
 
 dim3 grid_ffty(const Geo& G, int nrows, int nfields)
 {
@@ -2172,7 +2179,7 @@ dim3 grid_ffty(const Geo& G, int nrows, int nfields)
 
 dim3 grid_c2r(const Geo& G, int nrows, int nfields)
 {
-    const int L = pow2_kernel_size(G.nx) ? p2_lines(G.nx / 2) : FFT_L;
+    const int L = pow2_kernel_size(G.nx) ? p2_lines(G.nx / 2) : FFT_J;
     return dim3((G.ny + L - 1) / L, nrows, nfields);
 }
 
