@@ -1094,7 +1094,7 @@ __host__ __device__ constexpr int p2_stride_x(int n) { return p2_pad(n) + (p2_li
 
 // Divergence of the power-of-two path as its own streaming kernel
 // (divergence{2,4}, pressure.c:40-117).  A block owns an 8 (i) x 32 (j)
-// tile and climbs DV_KC planes.  Per plane, u with its x halo (rows i-2 ..
+// tile and climbs dv_planes planes.  Per plane, u with its x halo (rows i-2 ..
 // i+8) and v with its y halo (columns j-2 .. j+33, an even width) are staged
 // in shared memory by cp.async, double-buffered one plane ahead, so each
 // value crosses L2 once; for even ny the copies are 16-byte pairs that
@@ -1102,7 +1102,16 @@ __host__ __device__ constexpr int p2_stride_x(int n) { return p2_pad(n) + (p2_li
 // row loaded one plane ahead), and at the walls that window supplies the
 // extrapolated w of pressure.c:80-95.  The x transform then reads the
 // result as a real field.
-constexpr int DV_I = 8, DV_J = 32, DV_KC = 16;
+constexpr int DV_I = 8, DV_J = 32;
+// Planes per block: 16 where that gives 600 blocks (four per SM), else 4, so
+// that a small grid's planes are not walked one after another (with the x
+// transform, 64 x 64 x 64: 17 -> 12 us; 128 x 128 x 96, 384 tiles of 16
+// planes: 25.4 -> 22.9).
+__host__ __device__ inline int dv_planes(const Geo& G)
+{
+    const long long tiles = (long long) ((G.ny + DV_J - 1) / DV_J) * ((G.nx + DV_I - 1) / DV_I);
+    return tiles * ((G.nz + 15) / 16) >= 600 ? 16 : 4;
+}
 
 __device__ __forceinline__ void dv_cp8(double* dst, const double* src)
 {
@@ -1124,8 +1133,8 @@ __device__ __forceinline__ void k_div_body(const Geo& G, const DivArgs& A, uint3
     const int j0 = bid.x * DV_J, i0 = bid.y * DV_I;
     const int nx = G.nx, ny = G.ny, n2 = G.n2;
     const long long plane = G.plane;
-    const int k0 = GZ + bid.z * DV_KC;
-    const int k1 = min(k0 + DV_KC, n2 - GZ);
+    const int kc = dv_planes(G), k0 = GZ + bid.z * kc;
+    const int k1 = min(k0 + kc, n2 - GZ);
     const int i = i0 + ty, j = j0 + tx;
     const bool valid = i < nx && j < ny;
     // this thread's halo elements (even ny: one pair of u, one pair of v;
@@ -1899,7 +1908,7 @@ static void launch_r2c_p2(const Geo& G, const R2cArgs& A, int nrows, int nfields
 template <int N>
 static void launch_div_fftx_p2(const Geo& G, const DivArgs& A, cudaStream_t st)
 {
-    dim3 blk(DV_J, DV_I, 1), grd((G.ny + DV_J - 1) / DV_J, (G.nx + DV_I - 1) / DV_I, (G.nz + DV_KC - 1) / DV_KC);
+    dim3 blk(DV_J, DV_I, 1), grd((G.ny + DV_J - 1) / DV_J, (G.nx + DV_I - 1) / DV_I, (G.nz + dv_planes(G) - 1) / dv_planes(G));
     if (G.order == 2) k_div<2><<<grd, blk, 0, st>>>(G, A);
     else k_div<4><<<grd, blk, 0, st>>>(G, A);
     R2cArgs R{A.dv, A.spec, A.px, A.c8, GZ, 0, 0};
@@ -2160,7 +2169,7 @@ void launch_project(const Geo& G, const ProjArgs& A, cudaStream_t st)
 
 dim3 grid_div(const Geo& G)
 {
-    return dim3((G.ny + DV_J - 1) / DV_J, (G.nx + DV_I - 1) / DV_I, (G.nz + DV_KC - 1) / DV_KC);
+    return dim3((G.ny + DV_J - 1) / DV_J, (G.nx + DV_I - 1) / DV_I, (G.nz + dv_planes(G) - 1) / dv_planes(G));
 }
 
 dim3 grid_r2c(const Geo& G, int nrows, int nfields)

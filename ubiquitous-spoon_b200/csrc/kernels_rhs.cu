@@ -22,51 +22,52 @@ namespace cf {
 
 // ------------------------------------------------------------------ ghosts
 
-// One thread per column: wall ghost rows of u, v, c (apply_bc_u) and w
-// (apply_bc_w, then with EXTRAP the massflux4 extrapolation of
-// advect.c:100-131).
+// One thread per column and field (blockIdx.y: 0 u, 1 v, 2 c, 3 w): wall ghost
+// rows of u, v, c (apply_bc_u) and w (apply_bc_w, then with EXTRAP the
+// massflux4 extrapolation of advect.c:100-131).  Bound: latency, of one
+// column's few dependent reads and divisions; a thread per column doing the
+// four fields one after another took 8 us at 64 x 64 x 64, this 6.7.
 template <int ORDER, bool EXTRAP>
 __device__ __forceinline__ void ghosts_body(const Geo& G, const GhostArgs& A, uint3 bid)
 {
     long long col = (long long) bid.x * blockDim.x + threadIdx.x;
     if (col >= G.plane) return;
     const long long P = G.plane;
-    const int n2 = G.n2, kb = GZ - 1, kt = n2 - GZ;
-    auto at = [&](double* f, int k) -> double& { return f[(long long) k * P + col]; };
-    double* uf[3] = {A.F.u, A.F.v, A.F.c};
-    double bcb[3] = {A.bc_u, A.bc_v, A.bc_c_bot};
-    double bct[3] = {A.bc_u, A.bc_v, A.bc_c_top};
-    for (int q = 0; q < 3; q++) {
-        double* f = uf[q];
-        double g1, g2, g3;
-        bc_u_bot<ORDER>(A.ub, bcb[q], at(f, kb + 1), at(f, kb + 2), at(f, kb + 3), g1, g2, g3);
-        at(f, kb) = g1;
-        if (ORDER == 4) { at(f, kb - 1) = g2; at(f, kb - 2) = g3; }
-        bc_u_top<ORDER>(A.ut, bct[q], at(f, kt - 1), at(f, kt - 2), at(f, kt - 3), g1, g2, g3);
-        at(f, kt) = g1;
-        if (ORDER == 4) { at(f, kt + 1) = g2; at(f, kt + 2) = g3; }
+    const int n2 = G.n2, kb = GZ - 1, kt = n2 - GZ, q = bid.y;
+    if (q < 3) {
+        double* f = (q == 0 ? A.F.u : q == 1 ? A.F.v : A.F.c) + col;
+        auto at = [&](int k) -> double& { return f[k * P]; };
+        const double bcb = q == 0 ? A.bc_u : q == 1 ? A.bc_v : A.bc_c_bot;
+        const double bct = q == 0 ? A.bc_u : q == 1 ? A.bc_v : A.bc_c_top;
+        double b1, b2, b3, t1, t2, t3;
+        bc_u_bot<ORDER>(A.ub, bcb, at(kb + 1), at(kb + 2), at(kb + 3), b1, b2, b3);
+        bc_u_top<ORDER>(A.ut, bct, at(kt - 1), at(kt - 2), at(kt - 3), t1, t2, t3);
+        at(kb) = b1;
+        at(kt) = t1;
+        if (ORDER == 4) {
+            at(kb - 1) = b2;
+            at(kb - 2) = b3;
+            at(kt + 1) = t2;
+            at(kt + 2) = t3;
+        }
+        return;
     }
-    double* w = A.F.w;
+    double* w = A.F.w + col;
+    auto at = [&](int k) -> double& { return w[k * P]; };
     const int wt = n2 - GZ - 1;
-    double g1, g2, g3;
-    bc_w_bot<ORDER>(A.wb, A.bc_w, at(w, kb + 1), at(w, kb + 2), g1, g2, g3);
-    double top1, top2, top3;
-    bc_w_top<ORDER>(A.wt, A.bc_w, at(w, wt - 1), at(w, wt - 2), top1, top2, top3);
-    at(w, kb) = g1;
-    at(w, wt) = top1;
-    if (ORDER == 4 && EXTRAP) {
-        // massflux4 wall extrapolation (advect.c:108-109, 124-125)
-        at(w, kb - 1) = 2.0 * g1 - at(w, kb + 1);
-        at(w, kb - 2) = 2.0 * g1 - at(w, kb + 2);
-        at(w, wt + 1) = 2.0 * top1 - at(w, wt - 1);
-        at(w, wt + 2) = 2.0 * top1 - at(w, wt - 2);
-    } else if (ORDER == 4) {
-        at(w, kb - 1) = g2;
-        at(w, kb - 2) = g3;
-        at(w, wt + 1) = top2;
-        at(w, wt + 2) = top3;
+    const double x0 = at(kb + 1), x1 = at(kb + 2), y0 = at(wt - 1), y1 = at(wt - 2);
+    double b1, b2, b3, t1, t2, t3;
+    bc_w_bot<ORDER>(A.wb, A.bc_w, x0, x1, b1, b2, b3);
+    bc_w_top<ORDER>(A.wt, A.bc_w, y0, y1, t1, t2, t3);
+    at(kb) = b1;
+    at(wt) = t1;
+    if (ORDER == 4) {
+        // EXTRAP: massflux4 wall extrapolation (advect.c:108-109, 124-125)
+        at(kb - 1) = EXTRAP ? 2.0 * b1 - x0 : b2;
+        at(kb - 2) = EXTRAP ? 2.0 * b1 - x1 : b3;
+        at(wt + 1) = EXTRAP ? 2.0 * t1 - y0 : t2;
+        at(wt + 2) = EXTRAP ? 2.0 * t1 - y1 : t3;
     }
-    (void) g2; (void) g3; (void) top2; (void) top3;
 }
 
 template <int ORDER, bool EXTRAP>
@@ -636,20 +637,20 @@ __global__ void __launch_bounds__(RT_THREADS, RhsTile<ORDER>::BLOCKS) k_rhs_batc
 
 // ------------------------------------------------------------- launchers
 
-constexpr int GHOST_THREADS = 256;
+constexpr int GHOST_THREADS = 128;
 
-dim3 grid_ghosts(const Geo& G) { return dim3((unsigned) ((G.plane + GHOST_THREADS - 1) / GHOST_THREADS)); }
+dim3 grid_ghosts(const Geo& G) { return dim3((unsigned) ((G.plane + GHOST_THREADS - 1) / GHOST_THREADS), 4); }
 
 void launch_ghosts(const Geo& G, const GhostArgs& A, cudaStream_t st, bool extrap)
 {
     const int th = GHOST_THREADS;
-    const unsigned nb = grid_ghosts(G).x;
+    const dim3 nb = grid_ghosts(G);
     if (extrap) {
-        if (G.order == 2) k_ghosts<2, true><<<(unsigned) nb, th, 0, st>>>(G, A);
-        else k_ghosts<4, true><<<(unsigned) nb, th, 0, st>>>(G, A);
+        if (G.order == 2) k_ghosts<2, true><<<nb, th, 0, st>>>(G, A);
+        else k_ghosts<4, true><<<nb, th, 0, st>>>(G, A);
     } else {
-        if (G.order == 2) k_ghosts<2, false><<<(unsigned) nb, th, 0, st>>>(G, A);
-        else k_ghosts<4, false><<<(unsigned) nb, th, 0, st>>>(G, A);
+        if (G.order == 2) k_ghosts<2, false><<<nb, th, 0, st>>>(G, A);
+        else k_ghosts<4, false><<<nb, th, 0, st>>>(G, A);
     }
 }
 

@@ -330,7 +330,7 @@ __device__ __forceinline__ void line_chunks(const Geo& G, const SolveArgs& A, ui
 // computed.
 // Bound: HBM, 16 bytes per point and field; 1.47 ms for four fields at
 // 512 x 512 x 384 (4.4 TB/s).
-template <int ORDER, bool IS_W>
+template <int ORDER, bool IS_W, bool STATS>
 __device__ __forceinline__ void back_column(const Geo& G, const SolveArgs& A, uint3 bid)
 {
     constexpr int H = ORDER == 2 ? 1 : 3, PD = 4;
@@ -340,7 +340,6 @@ __device__ __forceinline__ void back_column(const Geo& G, const SolveArgs& A, ui
     const double* __restrict__ s = A.s + GZ * P + (valid ? col : 0);
     double* x = A.x + (valid ? col : 0);
     const double* __restrict__ rows = A.back;
-    const bool stats = A.partial != nullptr;
     const double* __restrict__ dz = G.dz + GZ;
     double y1 = 0.0, y2 = 0.0, y3 = 0.0, bulk = 0.0, p[PD];
 #pragma unroll
@@ -356,7 +355,7 @@ __device__ __forceinline__ void back_column(const Geo& G, const SolveArgs& A, ui
                 y -= __ldg(rows + i * H) * y1;   // y1 last
                 y3 = y2; y2 = y1; y1 = y;
                 if (valid) x[(GZ + i) * P] = y;
-                if (stats) bulk += y * __ldg(dz + i);
+                if (STATS) bulk += y * __ldg(dz + i);
             }
         }
     }
@@ -367,7 +366,7 @@ __device__ __forceinline__ void back_column(const Geo& G, const SolveArgs& A, ui
     double gb1, gb2, gt1, gt2;
     ghosts_bot<ORDER, IS_W>(A, x, P, valid, y1, y2, y3, gb1, gb2);
     ghosts_top<ORDER, IS_W>(A, x, P, n2, valid, top0, top1, top2, gt1, gt2);
-    if (!stats) return;
+    if (!STATS) return;
     const long long grp = col / 32;
     auto put = [&](int q, double v) {
         v = warp_sum(valid ? v : 0.0);
@@ -388,8 +387,8 @@ __device__ __forceinline__ void back_column(const Geo& G, const SolveArgs& A, ui
 
 // The control and its log row from the bulk mean, the averages of rows
 // g-2 .. g+1 (bot), n2-g-2 .. n2-g+1 (top) and the centreline.
-__device__ __forceinline__ void control_finish(const MassArgs& A, double mean, const double* bot, const double* top,
-                                               double centre)
+__device__ __forceinline__ void control_finish(const MassArgs& A, long long cnt, double mean, const double* bot,
+                                               const double* top, double centre)
 {
     const int g = GZ, n2 = A.n2;
     const double* dz = A.dz;
@@ -411,14 +410,12 @@ __device__ __forceinline__ void control_finish(const MassArgs& A, double mean, c
     for (int t = 0; t < 4; t++) s[t] += A.green[t] * m;
     *A.m_out = m;
     if (A.log_base) {
-        long long cnt = *A.counter;
         double* row = A.log_base + (cnt % A.log_cap) * LOG_COLS + A.col;
         row[0] = m;
         row[1] = s[1];
         row[2] = s[2];
         row[3] = s[0];
         row[4] = s[3];
-        if (A.advance) *A.counter = cnt + 1;
     }
 }
 
@@ -447,7 +444,9 @@ __device__ __forceinline__ void mass_control_body(const MassArgs& A)
         a += avg[k] * dz[k];
         l += dz[k];
     }
-    control_finish(A, a / l, avg + g - 2, avg + n2 - g - 2, 0.5 * (avg[g + (nz - 1) / 2] + avg[g + nz / 2]));
+    const long long cnt = *A.counter;
+    control_finish(A, cnt, a / l, avg + g - 2, avg + n2 - g - 2, 0.5 * (avg[g + (nz - 1) / 2] + avg[g + nz / 2]));
+    if (A.log_base && A.advance) *A.counter = cnt + 1;
 }
 __global__ void k_mass_control(MassArgs A)
 {
@@ -471,18 +470,29 @@ __device__ __forceinline__ void control_body(const ControlArgs& A, uint3 bid)
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x / 32] = v;
     __syncthreads();
-    if (threadIdx.x != 0) return;
-    v = 0.0;
-    for (int q = 0; q < CONTROL_THREADS / 32; q++) v += red[q];
-    A.sums[bid.x] = v * A.scale;
+    if (threadIdx.x >= 32) return;
+    unsigned done = 0;
+    if (threadIdx.x == 0) {
+        v = 0.0;
+        for (int q = 0; q < CONTROL_THREADS / 32; q++) v += red[q];
+        A.sums[bid.x] = v * A.scale;
+        __threadfence();
+        done = atomicAdd(A.ticket, 1u);
+    }
+    if (__shfl_sync(0xffffffffu, done, 0) != 2 * LINE_STATS - 1) return;
     __threadfence();
-    if (atomicAdd(A.ticket, 1u) != 2 * LINE_STATS - 1) return;
-    __threadfence();
-    *A.ticket = 0;   // for the next substep's launch
-    for (int q = 0; q < 2; q++) {
+    const long long cnt = *A.m[1].counter;   // both rows before the count moves on
+    __syncwarp();
+    if (threadIdx.x < 2) {
+        const int q = threadIdx.x;
         double s[LINE_STATS];
+#pragma unroll
         for (int e = 0; e < LINE_STATS; e++) s[e] = __ldcg(A.sums + q * LINE_STATS + e);
-        control_finish(A.m[q], s[0] * A.ilz, s + 1, s + 5, 0.5 * (s[9] + s[10]));
+        control_finish(A.m[q], cnt, s[0] * A.ilz, s + 1, s + 5, 0.5 * (s[9] + s[10]));
+    }
+    if (threadIdx.x == 0) {
+        *A.m[1].counter = cnt + 1;
+        *A.ticket = 0;   // for the next substep's launch
     }
 }
 
@@ -496,7 +506,7 @@ __global__ void __launch_bounds__(CONTROL_THREADS) k_control_batch(const BatchRe
 }
 
 // The line solves of the four fields in one launch; blockIdx.y selects the
-// field: 0 u, 1 v, 2 c, 3 w.  CHUNKS: both sweeps, partitioned; else the back
+// field: 0 u, 1 v, 2 c, 3 w (u and c with column sums).  CHUNKS: both sweeps, partitioned; else the back
 // sweep alone (line_partitioned decides).
 template <int ORDER, bool CHUNKS>
 __device__ __forceinline__ void line_body(const Geo& G, const SolveBatch& B, uint3 bid)
@@ -506,8 +516,9 @@ __device__ __forceinline__ void line_body(const Geo& G, const SolveBatch& B, uin
         if (bid.y < 3) line_chunks<ORDER, false>(G, B.a[bid.y], bid, line_sm);
         else line_chunks<ORDER, true>(G, B.a[3], bid, line_sm);
     } else {
-        if (bid.y < 3) back_column<ORDER, false>(G, B.a[bid.y], bid);
-        else back_column<ORDER, true>(G, B.a[3], bid);
+        if (bid.y == 3) back_column<ORDER, true, false>(G, B.a[3], bid);
+        else if (bid.y == 1) back_column<ORDER, false, false>(G, B.a[1], bid);
+        else back_column<ORDER, false, true>(G, B.a[bid.y], bid);
     }
 }
 
