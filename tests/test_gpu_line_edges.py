@@ -48,3 +48,29 @@ def test_substeps_match_restatement(cf, gpu, order, nx, ny, nz):
         bar = 1e-9 * np.maximum(np.abs(ref).max(axis=0), 1e-3)
         bar[[0, 5]] = np.maximum(bar[[0, 5]], 1e-14 / prm.dt)
         assert np.all(np.abs(log - ref) <= bar), np.abs(log - ref).max(axis=0)
+
+
+def test_batch_of_odd_and_even_planes_matches_plain(cf, gpu):
+    """A batch runs whole columns whatever the plain path does, odd and even
+    planes in launches of their own: against the plain path to rounding."""
+    out = []
+    for batched in (False, True):
+        insts = []
+        for q, (order, nx, ny, nz) in enumerate([(2, 12, 15, 10), (4, 10, 9, 12), (4, 12, 16, 20), (2, 48, 40, 33)]):
+            inst = cf.Instance(cf.Config.make(order, nx, ny, nz, 2 * np.pi, np.pi, 2.0, 1e-3, 1.0 / 3000.0, prandtl=0.71,
+                                              betg_y=0.05))
+            inst.init_fields(q, 0.1, 0.01)
+            insts.append(inst)
+        if batched:
+            cf.batch_step(insts, 6)
+        else:
+            for inst in insts:
+                inst.step(6)
+        for inst in insts:
+            inst.sync()
+        out.append([{nm: inst.get_field(nm, cf.LAYOUT_INTERIOR) for nm in "uvwcp"} for inst in insts])
+        for inst in insts:
+            inst.close()
+    for a, b in zip(*out):
+        for nm in "uvwcp":
+            assert np.linalg.norm(a[nm] - b[nm]) <= (1e-10 if nm == "p" else 1e-13) * np.linalg.norm(a[nm]), nm

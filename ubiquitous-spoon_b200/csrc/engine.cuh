@@ -289,7 +289,7 @@ dim3 grid_c2r(const Geo& G, int nrows, int nfields);
 dim3 grid_project(const Geo& G);
 bool batch_pow2(int n);                            // n has a power-of-two transform kernel
 void launch_ghosts_batch(const BatchLaunch& L, int order, cudaStream_t st);
-void launch_rhs_batch(const BatchLaunch& L, int order, cudaStream_t st);
+void launch_rhs_batch(const BatchLaunch& L, int key, cudaStream_t st);   // key: order, + 8 for odd ny
 void launch_line_batch(const BatchLaunch& L, int order, cudaStream_t st);
 void launch_control_batch(const BatchLaunch& L, cudaStream_t st);
 void launch_div_batch(const BatchLaunch& L, int order, cudaStream_t st);

@@ -1198,7 +1198,7 @@ void compile(const BatchSink& K, BatchProgram& P)
     for (const BatchStage& S : K.stages) {
         switch (S.kind) {
         case ST_GHOSTS: add_groups(P, BK_GHOSTS, S.ghosts, order, none); break;
-        case ST_RHS: add_groups(P, BK_RHS, S.rhs, order, none); break;
+        case ST_RHS: add_groups(P, BK_RHS, S.rhs, [](const auto& r) { return r.G.order + (r.G.ny % 2 ? 8 : 0); }, none); break;
         case ST_LINE: add_groups(P, BK_LINE, S.line, order, none, line_block(S.line)); break;
         case ST_CONTROL: add_groups(P, BK_CONTROL, S.control, none, none); break;
         case ST_DIV:

@@ -86,44 +86,67 @@ __global__ void k_ghosts_batch(const BatchRec<GhostArgs>* r, int n)
 
 // --------------------------------------------------------------------- RHS
 //
-// One block owns an 8 (x) by 32 (y) column tile and marches up its rows.
-// The 7 k-planes a row needs (k-3..k+3) of u, v, w, c, with a
-// periodic halo of 3 rows in x and 4 columns in y, sit in a ring of 8
-// shared-memory slots; the next plane streams in with cp.async while the
-// current row is computed.  Every
-// stencil value is read from shared memory.  Divisions by the grid metrics
-// are multiplications by their reciprocals (host tables), so results agree
+// One block owns an 8 (x) by 32 (y) column tile and marches up A.chunk rows.
+// Sixteen warps: four for each of u, v, w, c, a thread taking two
+// neighbouring points in y of its field.  A thread keeps its own column's next
+// values, the z fluxes carried up the column and the forward sweep; its
+// field's plane k with a periodic halo of 3 rows in x and 4 columns in y comes
+// from a ring of shared-memory planes, filled by cp.async one plane ahead, two
+// values per load.
+//
+// What one field's equation needs of another's are velocities interpolated
+// to its faces.  Each is formed once, by the thread that holds the values it
+// interpolates, and handed over through shared memory:
+//   u threads: u interpolated in y (for v's x flux) and in z (for w's)
+//   v threads: v interpolated in x (for u's y flux) and in z (for w's)
+//   w threads: w interpolated in x and y one row up (u's and v's z flux)
+// The faces of the tile's rim that no thread of the tile holds are formed by
+// the scalar's threads.  A row is: own differences and faces; a barrier; the
+// fluxes with the others' faces.  The face buffers alternate, so that one
+// block-wide barrier per row is enough.
+//
+// Bound: instruction issue and shared-memory bandwidth (order 4, ncu at
+// 256 x 256 x 192: LSU wavefronts 69 %, FP64 41 %, issue 54 %).  One thread
+// per point doing all four equations (256 threads, 253 registers) formed each
+// interpolated velocity four times and had two warps per scheduler to hide
+// latency with.  us, before and now: order 4 512 x 512 x 384 5161 -> 4390,
+// 256 x 256 x 192 748 -> 633, 128 x 128 x 96 (row blocks) 99 -> 89; order 2
+// 256 x 256 x 192 507 -> 478, 192 x 192 x 128 179 -> 168.
+// The four equations' loops have to fit the SM's instruction cache together
+// (about 27 KB at order 4): with two rows of points a thread, fewer
+// instructions but 42 KB of code, the warps waited for instructions (1105 us at
+// 256 x 256 x 192), and so they did with a test for odd ny and the wall
+// closures inside the loop (850).  Hence EVEN is a template parameter, the
+// interior rows have a loop of their own, and a scheduler's four warps all
+// work on the same field.
+//
+// Divisions by the grid metrics are multiplications by their reciprocals (host
+// tables), the 0.5 of a face average is folded into the interpolation weights
+// and a direction's metric is factored out of its flux sum, so results agree
 // with the reference to rounding, not bit for bit.
 //
-// After a row's four right-hand sides the same thread forms the right-hand
-// sides h of the four implicit solves (chanfast.c:459-480): the old field
-// window x_{k-H..k+H} is in the ring, f was just computed, g is read and
-// overwritten.
-// MODE RHS_SWEEP: it also runs that row of the solves' forward sweeps (the
-//   forward half of tridag/heptdag), leaving s; a block marches up all
-//   interior rows, and the back sweep follows in k_line (kernels_solve.cu).
-// MODE RHS_H: h itself is left; no row depends on the rows below it beyond the
-//   carried fluxes, so a block takes A.chunk rows of its tile (rhs_chunk),
-//   and both sweeps follow in k_line.
-// MODE RHS_CHANNEL (the fully implicit scheme of channel.c), rows as RHS_H: f
-//   has no x-y diffusion (channel.c:419-438) and h = x + nuadt (Lxy + Lz) x +
-//   gamdt f + zetdt g - hbc (channel.c:455-467, 531-543, 560-572, 636-648);
-//   A.nu and A.kappa then carry nuadt and nuadt / prandtl.  The spectral
-//   solves follow (kernels_pressure.cu).
-enum RhsMode { RHS_SWEEP, RHS_H, RHS_CHANNEL };
+// After a row's explicit right-hand side the thread forms the right-hand side
+// h of its implicit solve (chanfast.c:459-480), which overwrites g.
+// MODE RHS_SWEEP: and runs the solve's forward sweep, leaving s (the back
+//   sweep follows in k_line); the block takes the whole column.
+// MODE RHS_H: leaves h (both sweeps follow in k_line, partitioned).
+// MODE RHS_CHANNEL (the fully implicit scheme of channel.c): f has no x-y
+//   diffusion (channel.c:419-438) and h = x + nuadt (Lxy + Lz) x + gamdt f +
+//   zetdt g - hbc (channel.c:455-467, 531-543, 560-572, 636-648); A.nu and
+//   A.kappa then carry nuadt and nuadt / prandtl.  The spectral solves follow
+//   (kernels_pressure.cu).
 
 constexpr int RT_I = 8, RT_J = 32;
-constexpr int RT_THREADS = RT_I * RT_J;
+constexpr int RT_FIELD = RT_I * RT_J / 2;   // threads of one field
+constexpr int RT_THREADS = 4 * RT_FIELD;
+enum RhsMode { RHS_SWEEP, RHS_H, RHS_CHANNEL };
 
-// Ring geometry per order: the x-y halo and z reach of the stencils (order
-// 4: 3, the fourth-order fluxes and Laplacian; order 2: 2, the QUICK scalar
-// fluxes), a ring of the 2 ZH + 1 planes a row reads plus the one in flight
-// (8 and 6 slots).  Order 2 thus needs 83 KB of ring instead of 136 KB.
-// One block per SM for both: capping order 2 at 128 registers for two blocks
-// per SM measured 5-9 % slower (less instruction-level parallelism).
-// The y halo is rounded up to an even width (XL) so that, for even ny, every
-// haloed row segment starts on a 16-byte boundary in global and shared
-// memory: planes stream in as 16-byte copies that bypass L1.
+// Ring geometry per order: the x-y halo of the stencils (order 4: 3, the
+// fourth-order fluxes and Laplacian; order 2: 2, the QUICK scalar fluxes),
+// and a ring holding the ZH planes below and above a row and the one in
+// flight.  The y halo is rounded up to an even width (XL) so that, for even
+// ny, every haloed row segment starts on a 16-byte boundary in global and
+// shared memory.
 template <int ORDER>
 struct RhsTile {
     static constexpr int H = ORDER == 2 ? 2 : 3;
@@ -133,10 +156,6 @@ struct RhsTile {
     static constexpr int PI = RT_I + 2 * H, PJ = RT_J + 2 * XL;  // 14 x 40 / 12 x 36
     static constexpr int PLANE = PI * PJ;
     static constexpr int FIELD = SLOTS * PLANE;                  // one field's ring
-    static constexpr int LOADS = (PLANE + RT_THREADS - 1) / RT_THREADS;       // 8-byte copies per thread (odd ny)
-    static constexpr int PAIRS = PLANE / 2;
-    static constexpr int LOADS2 = (PAIRS + RT_THREADS - 1) / RT_THREADS;      // 16-byte copies per thread (even ny)
-    static constexpr int BLOCKS = 1;                             // launch bound: blocks per SM
     // plane kk >= 0 (every plane a row reads lies in 0 .. n2-1): an unsigned
     // remainder, a single AND for the 8-slot ring
     __host__ __device__ static constexpr int slot(int kk) { return (int) ((unsigned) kk % (unsigned) SLOTS); }
@@ -144,495 +163,544 @@ struct RhsTile {
 constexpr double B1h = 0.5 * B1, B2h = 0.5 * B2;   // halved interpolation weights (exact)
 // 7-point form of the fourth-order staggered second difference:
 // A1 (d+1/2 - d-1/2) + A2 (d+3/2 - d-3/2) = L1 (F1+F-1-2F0) + L2 (F2+F-2-2F0) + L3 (F3+F-3-2F0),
-// evaluated as L1 (F1+F-1) + L2 (F2+F-2) + L3 (F3+F-3) - 2 (L1+L2+L3) F0
+// evaluated as L1 (F1+F-1) + L2 (F2+F-2) + L3 (F3+F-3) - 2 (L1+L2+L3) F0.  Mathematically the
+// same; the centre term no longer cancels exactly, an error of a few ulps of |u| (1/dx^2 + 1/dy^2) nu.
 constexpr double L1 = A1 * A1 - 2.0 * A1 * A2, L2 = 2.0 * A1 * A2, L3 = A2 * A2;
 
-constexpr int RT_FWMAX = 14;   // widest fused forward row (order 4: 13), padded to 16-byte pairs
+constexpr int RT_FWMAX = 14;  // widest fused row (order 4: 13), padded to 16-byte pairs
 constexpr int RT_MROW = 12;   // per-row grid metrics: dydz[k-1..k+2], dxdz[k-1..k+2], ivol[k], ivolw[k] (+2 pad)
-// ring of haloed planes + two rows of each thread's g values + two rows of
-// the four fused coefficient rows + two rows of grid metrics
+// face buffers: u's with rows i0-2 .. i0+8, v's with columns j0-2 .. j0+33, w's on the tile
+constexpr int RF_U = (RT_I + 3) * RT_J, RF_V = RT_I * (RT_J + 4), RF_W = RT_I * RT_J;
+constexpr int RF_UY = 0, RF_UZ = RF_U, RF_VX = 2 * RF_U, RF_VZ = 2 * RF_U + RF_V, RF_WX = 2 * RF_U + 2 * RF_V,
+              RF_WY = RF_WX + RF_W, RF_ALL = RF_WY + RF_W;
+// ring of haloed planes + two rows of faces + per field two rows of its fused
+// coefficients and of the grid metrics + plane offsets of the copies
+template <int ORDER>
+__host__ __device__ constexpr int rhs_faces() { return 4 * RhsTile<ORDER>::FIELD; }
+template <int ORDER>
+__host__ __device__ constexpr int rhs_rows() { return rhs_faces<ORDER>() + 2 * RF_ALL; }
+template <int ORDER>
+__host__ __device__ constexpr int rhs_queue() { return rhs_rows<ORDER>() + 4 * 2 * (RT_FWMAX + RT_MROW); }
+template <int ORDER>
+__host__ __device__ constexpr int rhs_offs() { return rhs_queue<ORDER>() + (ORDER == 4 ? 4 * 2 * RT_THREADS : 0); }
 template <int ORDER>
 constexpr size_t rhs_smem_bytes()
 {
-    return (size_t) (4 * RhsTile<ORDER>::FIELD + 2 * 4 * RT_THREADS + 2 * 4 * RT_FWMAX + 2 * RT_MROW) * sizeof(double);
+    return (size_t) rhs_offs<ORDER>() * sizeof(double) + RhsTile<ORDER>::PLANE * sizeof(int);
 }
 
-// z fluxes of one advected field (order 4), carried up the column.  With
-// F1(k) = MZ(k) (Q(k) + Q(k+1)) / 2 and F3(k) = MZ(k+1) (Q(k) + Q(k+3)) / 2,
-// row k needs zph = F1(k), zmh = F1(k-1), zp3 = F3(k), zm3 = F3(k-3)
-// (advect.c:466-734), so each row forms one new mass flux MZ(k+1) and two
-// fluxes and takes the others from earlier rows; prime() forms the earlier
-// ones directly for the first row of a chunk.
-struct ZQueue {
-    double f1m, f3m[3], mzc, mz1, f1, f3;
-
-    // State as if row k-1 had just been processed (called at row k).
-    template <class QF, class MF>
-    __device__ __forceinline__ void prime(QF Q, MF MZ)
-    {
-        mz1 = MZ(0, 0, 0);
-        f1 = MZ(0, 0, -1) * 0.5 * (Q(0, 0, -1) + Q(0, 0, 0));
-        f3m[1] = MZ(0, 0, -2) * 0.5 * (Q(0, 0, -3) + Q(0, 0, 0));
-        f3m[2] = MZ(0, 0, -1) * 0.5 * (Q(0, 0, -2) + Q(0, 0, 1));
-        f3 = mz1 * 0.5 * (Q(0, 0, -1) + Q(0, 0, 2));
-    }
-
-    template <class QF, class MF>
-    __device__ __forceinline__ void advance(QF Q, MF MZ)
-    {
-        f1m = f1;
-        f3m[0] = f3m[1];
-        f3m[1] = f3m[2];
-        f3m[2] = f3;
-        mzc = mz1;
-        mz1 = MZ(0, 0, 1);
-        const double q0 = Q(0, 0, 0);
-        f1 = mzc * 0.5 * (q0 + Q(0, 0, 1));
-        f3 = mz1 * 0.5 * (q0 + Q(0, 0, 3));
-    }
-};
+extern __shared__ __align__(16) double rhs_sm[];
 
 __device__ __forceinline__ void cp_async8(double* dst, const double* src)
 {
     unsigned d = (unsigned) __cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src));
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async16(double* dst, const double* src)   // L2 only
 {
     unsigned d = (unsigned) __cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-template <int ORDER, int MODE>
-__device__ __forceinline__ void rhs_body(const Geo& G, const RhsArgs& A, uint3 bid)
+// pairs of points
+__device__ __forceinline__ double2 ld2(const double* p) { return *reinterpret_cast<const double2*>(p); }
+__device__ __forceinline__ void st2(double* p, double2 v) { *reinterpret_cast<double2*>(p) = v; }
+__device__ __forceinline__ double2 operator+(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ double2 operator-(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
+__device__ __forceinline__ double2 operator*(double2 a, double2 b) { return make_double2(a.x * b.x, a.y * b.y); }
+__device__ __forceinline__ double2 operator*(double a, double2 b) { return make_double2(a * b.x, a * b.y); }
+
+// Halved interpolation to the face between a0 and a1 (massflux{x,y,z}{2,4},
+// advect.c:6-283, with the 0.5 of the advected face value).
+template <int ORDER>
+__device__ __forceinline__ double2 face(double2 am, double2 a0, double2 a1, double2 a2)
 {
-    extern __shared__ double sm[];
-    using T = RhsTile<ORDER>;
-    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * RT_J + tx;
-    const int j0 = bid.x * RT_J, i0 = bid.y * RT_I;
-    const int nx = G.nx, ny = G.ny, n2 = G.n2;
-    const long long plane = (long long) nx * ny;
-    const int kb = GZ + (int) bid.z * A.chunk, ke = min(kb + A.chunk, GZ + G.nz);   // RHS_SWEEP: all interior rows, in order
+    if (ORDER == 2) return 0.25 * (a0 + a1);
+    return B1h * (a0 + a1) + B2h * (am + a2);
+}
 
-    // This thread's points (even ny: pairs of points) of a haloed plane,
-    // the same in every plane: their offsets within a field plane, computed
-    // once.  For even ny a pair starts at an even y index (j0 and XL are
-    // even), so it never straddles the periodic wrap and its global and
-    // shared addresses are 16-byte aligned.
-    const bool pairs = (ny & 1) == 0;
-    int goff[T::LOADS];
-#pragma unroll
-    for (int m = 0; m < T::LOADS; m++) {
-        const int r = tid + m * RT_THREADS;
-        int ii, jj;
-        if (pairs) { ii = r / (T::PJ / 2); jj = 2 * (r - ii * (T::PJ / 2)); }
-        else { ii = r / T::PJ; jj = r - ii * T::PJ; }
-        int gi = (i0 + ii - T::H) % nx; if (gi < 0) gi += nx;
-        int gj = (j0 + jj - T::XL) % ny; if (gj < 0) gj += ny;
-        goff[m] = gi * ny + gj;
-    }
+// Flux difference over a cell (advect{u,v,w}{2,4}, advect.c:286-734) from the
+// halved face velocities m[-2..1] and the advected values q[-3..3].
+template <int ORDER>
+__device__ __forceinline__ double2 flux(double2 mm2, double2 mm1, double2 m0, double2 m1, double2 qm3, double2 qm1,
+                                        double2 q0, double2 q1, double2 q3)
+{
+    const double2 d = m0 * (q0 + q1) - mm1 * (q0 + qm1);
+    if (ORDER == 2) return d;
+    return A1 * d + A2 * (m1 * (q0 + q3) - mm2 * (q0 + qm3));
+}
+
+struct RhsBlock {
+    int i0, j0, kb, ke, q, ty, jl;   // tile, rows, thread of the field, its row and first column
+    bool v0, v1;                     // this thread's points lie in the plane
+    long long plane, gij;            // gij: plane offset of the first point
+};
+
+// The march of field F's threads: 0 u, 1 v, 2 w, 3 c.
+template <int ORDER, int MODE, int F, bool EVEN>
+__device__ __forceinline__ void rhs_field(const Geo& G, const RhsArgs& A, const RhsBlock& T)
+{
+    using RT = RhsTile<ORDER>;
+    constexpr int PJ = RT::PJ, NZ = ORDER == 2 ? 2 : 3, HH = ORDER == 2 ? 1 : 3;   // z reach of the window, of the solve
+    constexpr int FWR = 2 * HH + 7;                               // fused row: cu[-HH..HH], cf, cg, c0, f1, f2, f3
+    const int n2 = G.n2, top = n2 - GZ - 1;                       // last interior row
+    const double* __restrict__ src = F == 0 ? A.u : F == 1 ? A.v : F == 2 ? A.w : A.c;
+    double* __restrict__ fout = (F == 0 ? A.fu : F == 1 ? A.fv : F == 2 ? A.fw : A.fc) + T.gij + T.kb * T.plane;   // row k
+    double* gio = A.sw[F].g + T.gij + T.kb * T.plane;                                                             // row k
+    double* const mine = rhs_sm + F * RT::FIELD;
+    const int* const goff = reinterpret_cast<const int*>(rhs_sm + rhs_offs<ORDER>());   // plane offsets of the copies
+    const int at = (T.ty + RT::H) * PJ + T.jl + RT::XL;           // own point within a plane
+    const double2 z2 = make_double2(0.0, 0.0);
+
+    // ---- copies: this field's planes, coefficients and metrics
+    const double* b = src + (T.kb - RT::ZH) * T.plane;   // the next plane to copy
     auto load_plane = [&](int kk) {
-        const long long base = (long long) kk * plane;   // same for the whole block
-        const double* bu = A.u + base;
-        const double* bv = A.v + base;
-        const double* bw = A.w + base;
-        const double* bc = A.c + base;
-        double* ps = sm + T::slot(kk) * T::PLANE;
-        if (pairs) {
+        double* d = mine + RT::slot(kk) * RT::PLANE;
+        if (EVEN) {   // pairs
 #pragma unroll
-            for (int m = 0; m < T::LOADS2; m++) {
-                if (tid + m * RT_THREADS < T::PAIRS) {
-                    double* d = ps + 2 * (tid + m * RT_THREADS);
-                    const int o = goff[m];
-                    cp_async16(d, bu + o);
-                    cp_async16(d + T::FIELD, bv + o);
-                    cp_async16(d + 2 * T::FIELD, bw + o);
-                    cp_async16(d + 3 * T::FIELD, bc + o);
-                }
-            }
+            for (int e = 0; e < RT::PLANE / 2; e += RT_FIELD)
+                if (e + RT_FIELD <= RT::PLANE / 2 || e + T.q < RT::PLANE / 2)
+                    cp_async16(d + 2 * (e + T.q), b + goff[e + T.q]);
         } else {
 #pragma unroll
-            for (int m = 0; m < T::LOADS; m++) {
-                if (tid + m * RT_THREADS < T::PLANE) {
-                    double* d = ps + tid + m * RT_THREADS;
-                    const int o = goff[m];
-                    cp_async8(d, bu + o);
-                    cp_async8(d + T::FIELD, bv + o);
-                    cp_async8(d + 2 * T::FIELD, bw + o);
-                    cp_async8(d + 3 * T::FIELD, bc + o);
-                }
-            }
+            for (int e = 0; e < RT::PLANE; e += RT_FIELD)
+                if (e + RT_FIELD <= RT::PLANE || e + T.q < RT::PLANE) cp_async8(d + e + T.q, b + goff[e + T.q]);
         }
-        cp_async_commit();
+        b += T.plane;
     };
-    // g values (per thread) and fused coefficient rows (per block) of row kk,
-    // staged one row ahead so the sweeps never wait on global memory
-    double* gst = sm + 4 * T::FIELD;              // [2][4][RT_THREADS]
-    double* cst = gst + 2 * 4 * RT_THREADS;       // [2][4][RT_FWMAX]
-    double* mst = cst + 2 * 4 * RT_FWMAX;         // [2][RT_MROW]
-    constexpr int FWR = (ORDER == 2 ? 3 : 7) + 6; // fused row width (host_band.h fused_rows)
-    const long long gij = (i0 + ty < nx && j0 + tx < ny) ? (long long) (i0 + ty) * ny + (j0 + tx) : 0;
-    auto load_extras = [&](int kk) {
-        const long long o = (long long) kk * plane + gij;
-        double* d = gst + (kk & 1) * 4 * RT_THREADS + tid;
-#pragma unroll
-        for (int f = 0; f < 4; f++) cp_async8(d + f * RT_THREADS, A.sw[f].g + o);
-        if (tid < 4 * FWR) {
-            const int f = tid / FWR, e = tid - f * FWR;
-            if (!(f == 2 && kk - GZ >= G.nz - 1))   // the w solve has nz - 1 rows
-                cp_async8(cst + ((kk & 1) * 4 + f) * RT_FWMAX + e, A.sw[f].rows + (kk - GZ) * FWR + e);
-        }
-        const int e = tid - 4 * FWR;   // grid metrics of row kk (rows kk-1 .. kk+2 lie within 0 .. n2-1)
-        if (e >= 0 && e < 10) {
-            const double* src = e < 4 ? G.dydz + kk - 1 + e : e < 8 ? G.dxdz + kk - 5 + e : e == 8 ? G.ivol + kk : G.ivolw + kk;
-            cp_async8(mst + (kk & 1) * RT_MROW + e, src);
-        }
+    double* const cst = rhs_sm + rhs_rows<ORDER>() + F * 2 * (RT_FWMAX + RT_MROW);   // [2][RT_FWMAX] fused coefficients
+    double* const mst = cst + 2 * RT_FWMAX;                      // [2][RT_MROW] grid metrics
+    // thread e copies value e of a row: its coefficients, then the metrics
+    // (rows kk-1 .. kk+2 lie within 0 .. n2-1)
+    const double* xsrc = nullptr;
+    int xstep = 0, xdst = 0;
+    if (T.q < FWR) {
+        xsrc = A.sw[F].rows + (T.kb - GZ) * FWR + T.q;
+        xstep = FWR;
+        xdst = T.q;
+    } else if (T.q >= 32 && T.q < 42) {
+        const int m = T.q - 32;
+        xsrc = m < 4 ? G.dydz + T.kb - 1 + m : m < 8 ? G.dxdz + T.kb - 5 + m : m == 8 ? G.ivol + T.kb : G.ivolw + T.kb;
+        xstep = 1;
+        xdst = 2 * RT_FWMAX + m;
+    }
+    const int xodd = T.q < FWR ? RT_FWMAX : RT_MROW;
+    auto load_extras = [&](int kk) {   // (the w solve has nz - 1 rows)
+        if (xsrc && !(F == 2 && T.q < FWR && kk >= top)) cp_async8(cst + xdst + (kk & 1) * xodd, xsrc);
+        xsrc = xsrc ? xsrc + xstep : xsrc;
     };
-    load_extras(kb);
-    for (int kk = kb - T::ZH; kk <= kb + T::ZH; kk++) load_plane(kk);
+    auto load_g = [&](int kk, const double* p) {
+        if (F == 2 && kk >= top) return z2;
+        if (EVEN) return T.v0 ? ld2(p) : z2;
+        return make_double2(T.v0 ? p[0] : 0.0, T.v1 ? p[1] : 0.0);
+    };
+    load_extras(T.kb);
+    for (int kk = T.kb - RT::ZH; kk <= T.kb + RT::ZH; kk++) load_plane(kk);
+    double2 gnext = load_g(T.kb, gio);
     cp_async_wait_all();
     __syncthreads();
 
-    const int i = i0 + ty, j = j0 + tx;
-    const bool out = i < nx && j < ny;
-    const double dxdy = G.dxdy, idx = G.idx, idy = G.idy;
-    const double idx2 = idx * idx, idy2 = idy * idy;
-    const double lapc = -2.0 * (L1 + L2 + L3) * (idx2 + idy2);   // centre weight of the sum-form Laplacian
-    const int kb_w = GZ - 1, kt_u = n2 - GZ;   // wall ghost rows of cell-centred fields
-
-    int k = kb;
-    auto at = [&](int f, int di, int dj, int dk) -> double {
-        return sm[f * T::FIELD + T::slot(k + dk) * T::PLANE + (ty + T::H + di) * T::PJ + (tx + T::XL + dj)];
-    };
-    auto U = [&](int di, int dj, int dk) { return at(0, di, dj, dk); };
-    auto V = [&](int di, int dj, int dk) { return at(1, di, dj, dk); };
-    auto W = [&](int di, int dj, int dk) { return at(2, di, dj, dk); };
-    auto C = [&](int di, int dj, int dk) { return at(3, di, dj, dk); };
-
-    // grid metrics of the current row, staged one row ahead: dydz[k+dk],
-    // dxdz[k+dk] for dk = -1 .. 2, 1 / cell volume, 1 / w-face volume
-    auto DYDZ = [&](int dk) { return mst[(k & 1) * RT_MROW + 1 + dk]; };
-    auto DXDZ = [&](int dk) { return mst[(k & 1) * RT_MROW + 5 + dk]; };
-    // massflux{x,y,z}4 (advect.c:88-283): fourth-order interpolation of the
-    // w mass fluxes (the u and v ones are formed per face below)
-    auto mx_w = [&](int di, int dj, int dk) {
-        return B1 * (dxdy * W(di, dj, dk) + dxdy * W(di + 1, dj, dk)) + B2 * (dxdy * W(di - 1, dj, dk) + dxdy * W(di + 2, dj, dk)); };
-    auto my_w = [&](int di, int dj, int dk) {
-        return B1 * (dxdy * W(di, dj, dk) + dxdy * W(di, dj + 1, dk)) + B2 * (dxdy * W(di, dj - 1, dk) + dxdy * W(di, dj + 2, dk)); };
-    auto mz_w = [&](int di, int dj, int dk) {
-        return B1 * (dxdy * W(di, dj, dk) + dxdy * W(di, dj, dk + 1)) + B2 * (dxdy * W(di, dj, dk - 1) + dxdy * W(di, dj, dk + 2)); };
-    // massflux{x,y,z}2 (advect.c:6-85)
-    auto mx_u2 = [&](int di, int dj, int dk) { double d = DYDZ(dk); return 0.5 * (d * U(di, dj, dk) + d * U(di + 1, dj, dk)); };
-    auto mx_v2 = [&](int di, int dj, int dk) { double d = DXDZ(dk); return 0.5 * (d * V(di, dj, dk) + d * V(di + 1, dj, dk)); };
-    auto mx_w2 = [&](int di, int dj, int dk) { return 0.5 * (dxdy * W(di, dj, dk) + dxdy * W(di + 1, dj, dk)); };
-    auto my_u2 = [&](int di, int dj, int dk) { double d = DYDZ(dk); return 0.5 * (d * U(di, dj, dk) + d * U(di, dj + 1, dk)); };
-    auto my_v2 = [&](int di, int dj, int dk) { double d = DXDZ(dk); return 0.5 * (d * V(di, dj, dk) + d * V(di, dj + 1, dk)); };
-    auto my_w2 = [&](int di, int dj, int dk) { return 0.5 * (dxdy * W(di, dj, dk) + dxdy * W(di, dj + 1, dk)); };
-    auto mz_u2 = [&](int di, int dj, int dk) { return 0.5 * (DYDZ(dk) * U(di, dj, dk) + DYDZ(dk + 1) * U(di, dj, dk + 1)); };
-    auto mz_v2 = [&](int di, int dj, int dk) { return 0.5 * (DXDZ(dk) * V(di, dj, dk) + DXDZ(dk + 1) * V(di, dj, dk + 1)); };
-    auto mz_w2 = [&](int di, int dj, int dk) { return 0.5 * (dxdy * W(di, dj, dk) + dxdy * W(di, dj, dk + 1)); };
-
-    const double qk = -0.125;   // QUICK coefficient (scalar.c:79-162)
-    // The face value between cells c0 and c1 takes the upwind curvature
-    // x - 2y + z of (c1, c0, c-1) for m > 0, else of (c2, c1, c0): the
-    // curvature centred on the upwind cell.  Each point forms the curvatures
-    // of cells i-1, i, i+1 once per direction and both faces pick theirs.
-    auto curv = [](double x, double y, double z) { return x - 2.0 * y + z; };
-    auto quick = [&](double m, double c0, double c1, double kup, double kdn) {
-        double cph = 0.5 * (c0 + c1);
-        cph += qk * (m > 0.0 ? kup : kdn);
-        return m * cph;
-    };
-    // add_buoyancy is skipped when every betg is zero (adding exact zeros)
+    auto ringat = [&](int f, int kk) { return rhs_sm + f * RT::FIELD + RT::slot(kk) * RT::PLANE + at; };
+    const double dxdy = G.dxdy, idx2 = G.idx * G.idx, idy2 = G.idy * G.idy;
+    const double diff = F == 3 ? A.kappa : A.nu;
     const bool buoyancy = A.betg_x != 0.0 || A.betg_y != 0.0 || A.betg_z != 0.0;
+    const double shift = A.sw[F].gshift ? *A.sw[F].gshift : 0.0;
 
-    // z fluxes carried up the column: the queues and the scalar flux
-    // through the bottom face, primed for the first row.
-    ZQueue zq_u{}, zq_v{}, zq_w{};
-    if (ORDER == 4) {
-        zq_u.prime(U, mx_w);
-        zq_v.prime(V, my_w);
-        zq_w.prime(W, mz_w);
+    // w interpolated to this point's u (v) face in plane kk, from the ring
+    auto wface = [&](int kk) {
+        const double* w = ringat(2, kk);
+        if (F == 0) return face<ORDER>(ORDER == 4 ? ld2(w - PJ) : z2, ld2(w), ld2(w + PJ), ORDER == 4 ? ld2(w + 2 * PJ) : z2);
+        const double2 a = ld2(w - 2), b = ld2(w), c = ld2(w + 2);
+        return face<ORDER>(make_double2(a.y, b.x), b, make_double2(b.y, c.x), c);
+    };
+
+    // ---- state carried up the column, as if row kb - 1 had just been done
+    // own values of rows k-LO .. k+NZ.  At order 4 the rows below k are read back
+    // from the ring: kept, they cost 12 registers (spills with the sweep) and as
+    // many moves a row, 4517 against 4390 us at 512 x 512 x 384; at order 2,
+    // with registers to spare, keeping them is the faster way, 478 against 496
+    // us at 256 x 256 x 192.
+    constexpr int LO = ORDER == 2 ? NZ : 0;
+    double2 zw[LO + NZ + 1];
+#pragma unroll
+    for (int d = 0; d < LO + NZ; d++) zw[d + 1] = ld2(ringat(F, T.kb - LO + d));
+    zw[0] = z2;
+    // z fluxes with the halved face velocity m(k): F1(k) = m(k) (q(k) + q(k+1)),
+    // F3(k) = m(k+1) (q(k) + q(k+3)); row k needs F1(k), F1(k-1), F3(k), F3(k-3)
+    double2 f1 = z2, mz = z2;   // F1(k-1), m(k); F3 of the last rows in this thread's own slots f3q[k & 3]
+    double* const f3q = rhs_sm + rhs_queue<ORDER>() + 2 * threadIdx.x;
+    double2 kz = z2, fz = z2;                                 // scalar: z curvature of row k, flux of face k-1
+    if (F < 3) {
+        auto own = [&](int d) { return ld2(ringat(F, T.kb + d)); };
+        double2 mm1, mm2 = z2;
+        if (F == 2) {
+            mm1 = face<ORDER>(ORDER == 4 ? own(-2) : z2, own(-1), own(0), ORDER == 4 ? own(1) : z2);
+            if (ORDER == 4) {
+                mz = face<ORDER>(own(-1), own(0), own(1), own(2));
+                mm2 = face<ORDER>(own(-3), own(-2), own(-1), own(0));
+            }
+        } else {
+            mm1 = wface(T.kb - 1);
+            if (ORDER == 4) {
+                mz = wface(T.kb);
+                mm2 = wface(T.kb - 2);
+            }
+        }
+        f1 = mm1 * (own(-1) + own(0));
+        if (ORDER == 4) {
+            st2(f3q + ((T.kb - 3) & 3) * 2 * RT_THREADS, mm2 * (own(-3) + own(0)));
+            st2(f3q + ((T.kb - 2) & 3) * 2 * RT_THREADS, mm1 * (own(-2) + own(1)));
+            st2(f3q + ((T.kb - 1) & 3) * 2 * RT_THREADS, mz * (own(-1) + own(2)));
+        }
     }
-    // z curvature of cell k (carried from row to row) and the scalar flux
-    // through the bottom face of the first row
-    double kz = curv(C(0, 0, 1), C(0, 0, 0), C(0, 0, -1));
-    double fzp_prev = quick(dxdy * W(0, 0, -1), C(0, 0, -1), C(0, 0, 0), curv(C(0, 0, 0), C(0, 0, -1), C(0, 0, -2)), kz);
+    auto curv = [](double2 x, double2 y, double2 z) { return x - 2.0 * y + z; };
+    // QUICK (scalar.c:79-162): the face value between c0 and c1 takes the
+    // curvature centred on the upwind cell
+    auto quick = [](double2 m, double2 c0, double2 c1, double2 kup, double2 kdn) {
+        const double2 k = make_double2(m.x > 0.0 ? kup.x : kdn.x, m.y > 0.0 ? kup.y : kdn.y);
+        return m * (0.5 * (c0 + c1) + -0.125 * k);
+    };
+    if (F == 3) {
+        const double2 cm2 = ld2(ringat(F, T.kb - 2)), cm1 = ld2(ringat(F, T.kb - 1)), c0 = zw[LO + 1], c1 = zw[LO + 2];
+        kz = curv(c1, c0, cm1);
+        fz = quick(dxdy * ld2(ringat(2, T.kb - 1)), cm1, c0, curv(c0, cm1, cm2), kz);
+    }
+    double2 s1 = z2, s2 = z2, s3 = z2;   // forward sweep: s of rows k-1, k-2, k-3
 
-    // Forward-sweep state: s of rows k-1, k-2, k-3 per field, the lazily
-    // applied shifts of g (u: mdpdx, c: dcdt of the previous control step),
-    // and the ghost values of the old w below / above its wall faces
-    // (apply_bc_w; the ring holds the massflux4 extrapolation there instead).
-    constexpr int H = ORDER == 2 ? 1 : 3;
-    double su1 = 0.0, su2 = 0.0, su3 = 0.0, sv1 = 0.0, sv2 = 0.0, sv3 = 0.0;
-    double sw1 = 0.0, sw2 = 0.0, sw3 = 0.0, sc1 = 0.0, sc2 = 0.0, sc3 = 0.0;
-    const double shift_u = A.sw[0].gshift ? *A.sw[0].gshift : 0.0;
-    const double shift_c = A.sw[3].gshift ? *A.sw[3].gshift : 0.0;
-    double gb0, gb1, gb2, gt0 = 0.0, gt1 = 0.0, gt2 = 0.0;
-    bc_w_bot<ORDER>(A.wbot, A.wbc_bot, W(0, 0, 0), W(0, 0, 1), gb0, gb1, gb2);
-    (void) gb0;
-    auto sweep = [&](int f, auto X, double fk, double gk, double lk, double& s1, double& s2, double& s3) {
-        // staged coefficient row, read as 16-byte pairs (same value for the
-        // whole block: broadcast loads)
-        const double2* r2 = reinterpret_cast<const double2*>(cst + ((k & 1) * 4 + f) * RT_FWMAX);
+    auto row = [&](int k, auto wall_tag) {
+        constexpr bool WALL = decltype(wall_tag)::value;   // rows within two of a wall
+        const bool live = F != 2 || !WALL || k < top;      // w has no point on the top wall
+        double* const fb = rhs_sm + rhs_faces<ORDER>() + (k & 1) * RF_ALL;
+        const double* mrow = mst + (k & 1) * RT_MROW;
+        auto DYDZ = [&](int d) { return mrow[1 + d]; };
+        auto DXDZ = [&](int d) { return mrow[5 + d]; };
+        // the window moves up one row
+#pragma unroll
+        for (int d = 0; d < LO + NZ; d++) zw[d] = zw[d + 1];
+        zw[LO + NZ] = ld2(ringat(F, k + NZ));
+        auto Z = [&](int d) { return LO + d >= 0 ? zw[LO + d >= 0 ? LO + d : 0] : ld2(ringat(F, k + d)); };
+        const double2 q0 = Z(0);
+        const double2 gk = make_double2(gnext.x + shift, gnext.y + shift);
+        if (k + 1 < T.ke) gnext = load_g(k + 1, gio + T.plane);
+
+        // ---- plane k: x neighbours, y neighbours (columns j-4 .. j+5)
+        const double* p = ringat(F, k);
+        double2 x[7], y[5];
+#pragma unroll
+        for (int d = -3; d <= 3; d++) x[d + 3] = d == 0 ? q0 : (ORDER == 4 || (d >= -2 && d <= 2)) ? ld2(p + d * PJ) : z2;
+#pragma unroll
+        for (int d = -2; d <= 2; d++) y[d + 2] = d == 0 ? q0 : (ORDER == 4 || (d >= -1 && d <= 1)) ? ld2(p + 2 * d) : z2;
+        auto X = [&](int d) { return x[d + 3]; };
+        // (q(j + d), q(j + 1 + d))
+        auto Y = [&](int d) {
+            const int e = d + 4;
+            return (e & 1) == 0 ? y[e / 2] : make_double2(y[(e - 1) / 2].y, y[(e + 1) / 2].x);
+        };
+        // add_laplacexy_operator_{u,w}{2,4} (diffuseu.c:286-359, diffusew.c:290-363)
+        double2 lap;
+        if (ORDER == 2) {
+            lap = diff * (idx2 * (X(1) - 2.0 * q0 + X(-1)) + idy2 * (Y(1) - 2.0 * q0 + Y(-1)));
+        } else {
+            const double lapc = -2.0 * (L1 + L2 + L3) * (idx2 + idy2);
+            const double2 lx = L3 * (X(3) + X(-3)) + L2 * (X(2) + X(-2)) + L1 * (X(1) + X(-1));
+            const double2 ly = L3 * (Y(3) + Y(-3)) + L2 * (Y(2) + Y(-2)) + L1 * (Y(1) + Y(-1));
+            lap = diff * ((idx2 * lx + idy2 * ly) + lapc * q0);
+        }
+
+        // ---- faces for the other fields, and the flux of the field's own direction
+        const int wat = T.ty * RT_J + T.jl, uat = (T.ty + 2) * RT_J + T.jl, vat = T.ty * (RT_J + 4) + T.jl + 2;
+        double2 own = z2;
+        if (F == 0) {
+            st2(fb + RF_UY + uat, face<ORDER>(Y(-1), q0, Y(1), Y(2)));
+            if (ORDER == 2) st2(fb + RF_UZ + uat, 0.25 * (DYDZ(0) * q0 + DYDZ(1) * Z(1)));
+            else st2(fb + RF_UZ + uat, (B1h * DYDZ(0)) * q0 + (B1h * DYDZ(1)) * Z(1) + ((B2h * DYDZ(-1)) * Z(-1) + (B2h * DYDZ(2)) * Z(2)));
+            own = flux<ORDER>(ORDER == 4 ? face<ORDER>(X(-3), X(-2), X(-1), q0) : z2, face<ORDER>(X(-2), X(-1), q0, X(1)),
+                              face<ORDER>(X(-1), q0, X(1), X(2)), ORDER == 4 ? face<ORDER>(q0, X(1), X(2), X(3)) : z2,
+                              X(-3), X(-1), q0, X(1), X(3));
+        } else if (F == 1) {
+            st2(fb + RF_VX + vat, face<ORDER>(X(-1), q0, X(1), X(2)));
+            if (ORDER == 2) st2(fb + RF_VZ + vat, 0.25 * (DXDZ(0) * q0 + DXDZ(1) * Z(1)));
+            else st2(fb + RF_VZ + vat, (B1h * DXDZ(0)) * q0 + (B1h * DXDZ(1)) * Z(1) + ((B2h * DXDZ(-1)) * Z(-1) + (B2h * DXDZ(2)) * Z(2)));
+            // faces j-2 .. j+2, each once for both points
+            const double2 e0 = face<ORDER>(Y(-3), Y(-2), Y(-1), q0);                     // faces -2, -1
+            const double2 e2 = face<ORDER>(Y(-1), q0, Y(1), Y(2));                       // faces 0, 1
+            const double e4 = ORDER == 4 ? B1h * (Y(2).x + Y(3).x) + B2h * (Y(1).x + Y(3).y) : 0.0;   // face 2
+            own = flux<ORDER>(e0, make_double2(e0.y, e2.x), e2, make_double2(e2.y, e4), Y(-3), Y(-1), q0, Y(1), Y(3));
+        } else if (F == 2) {
+            if (ORDER == 2) {   // plane k: the z fluxes use m(k)
+                st2(fb + RF_WX + wat, 0.25 * (q0 + X(1)));
+                st2(fb + RF_WY + wat, 0.25 * (q0 + Y(1)));
+            } else {            // plane k + 1: they use m(k + 1)
+                const double* w = ringat(2, k + 1);
+                const double2 w0 = Z(1), a = ld2(w - 2), c = ld2(w + 2);
+                st2(fb + RF_WX + wat, face<ORDER>(ld2(w - PJ), w0, ld2(w + PJ), ld2(w + 2 * PJ)));
+                st2(fb + RF_WY + wat, face<ORDER>(make_double2(a.y, w0.x), w0, make_double2(w0.y, c.x), c));
+            }
+        } else {
+            // the rim: u's faces of rows i0-2, i0-1, i0+8 (order 2: i0-1), v's of the
+            // column pairs j0-2 and j0+32 (order 2: j0-2)
+            if (ORDER == 4 ? T.q < 48 : T.q < 16) {
+                const int r = ORDER == 2 ? -1 : T.q < 16 ? -2 : T.q < 32 ? -1 : RT_I, j = 2 * (T.q & 15);
+                const int o = (r + RT::H) * PJ + j + RT::XL;
+                auto U = [&](int kk) { return rhs_sm + RT::slot(kk) * RT::PLANE + o; };
+                const double* u = U(k);
+                const double2 a = ld2(u - 2), b = ld2(u), c = ld2(u + 2);
+                double* d = fb + RF_UY + (r + 2) * RT_J + j;
+                st2(d, face<ORDER>(make_double2(a.y, b.x), b, make_double2(b.y, c.x), c));
+                const double2 b1 = ld2(U(k + 1));
+                if (ORDER == 2) st2(d + RF_UZ - RF_UY, 0.25 * (DYDZ(0) * b + DYDZ(1) * b1));
+                else st2(d + RF_UZ - RF_UY, (B1h * DYDZ(0)) * b + (B1h * DYDZ(1)) * b1
+                                            + ((B2h * DYDZ(-1)) * ld2(U(k - 1)) + (B2h * DYDZ(2)) * ld2(U(k + 2))));
+            } else if (ORDER == 4 ? T.q < 64 : T.q >= 32 && T.q < 40) {
+                const int e = T.q - (ORDER == 4 ? 48 : 32);
+                const int r = ORDER == 4 ? e >> 1 : e, j = ORDER == 4 && (e & 1) ? RT_J : -2;
+                const int o = RT::FIELD + (r + RT::H) * PJ + j + RT::XL;
+                auto V = [&](int kk) { return rhs_sm + RT::slot(kk) * RT::PLANE + o; };
+                const double* v = V(k);
+                const double2 b = ld2(v), b1 = ld2(V(k + 1));
+                double* d = fb + RF_VX + r * (RT_J + 4) + j + 2;
+                st2(d, face<ORDER>(ORDER == 4 ? ld2(v - PJ) : z2, b, ld2(v + PJ), ORDER == 4 ? ld2(v + 2 * PJ) : z2));
+                if (ORDER == 2) st2(d + RF_VZ - RF_VX, 0.25 * (DXDZ(0) * b + DXDZ(1) * b1));
+                else st2(d + RF_VZ - RF_VX, (B1h * DXDZ(0)) * b + (B1h * DXDZ(1)) * b1
+                                            + ((B2h * DXDZ(-1)) * ld2(V(k - 1)) + (B2h * DXDZ(2)) * ld2(V(k + 2))));
+            }
+        }
+
+        double2 f;
+        if (F == 3) {   // flux_quick + advect_scalar (scalar.c:79-162): no faces of others
+            const double* u = ringat(0, k);
+            const double* v = ringat(1, k);
+            const double2 va = ld2(v - 2), vb = ld2(v);
+            const double2 kx0 = curv(X(1), q0, X(-1)), ky0 = curv(Y(1), q0, Y(-1)), kzp = curv(Z(2), Z(1), q0);
+            const double2 fxp = quick(DYDZ(0) * ld2(u), q0, X(1), kx0, curv(X(2), X(1), q0));
+            const double2 fxm = quick(DYDZ(0) * ld2(u - PJ), X(-1), q0, curv(q0, X(-1), X(-2)), kx0);
+            const double2 fyp = quick(DXDZ(0) * vb, q0, Y(1), ky0, curv(Y(2), Y(1), q0));
+            const double2 fym = quick(DXDZ(0) * make_double2(va.y, vb.x), Y(-1), q0, curv(q0, Y(-1), Y(-2)), ky0);
+            const double2 fzp = quick(dxdy * ld2(ringat(2, k)), q0, Z(1), kz, kzp);
+            f = (-mrow[8]) * ((fxp - fxm) + (fyp - fym) + (fzp - fz));
+            kz = kzp;
+            fz = fzp;
+        }
+        __syncthreads();   // the row's faces are in place
+
+        if (F < 3) {
+            double2 other;   // the flux (for w: both) of the directions whose faces others hold
+            if (F == 0 || F == 2) {   // y flux with v's faces, columns j-2 .. j+3
+                const double* m = fb + (F == 0 ? RF_VX : RF_VZ) + vat;
+                const double2 a = ld2(m - 2), b = ld2(m), c = ORDER == 4 ? ld2(m + 2) : z2;
+                other = flux<ORDER>(a, make_double2(a.y, b.x), b, make_double2(b.y, c.x), Y(-3), Y(-1), q0, Y(1), Y(3));
+            }
+            if (F == 1 || F == 2) {   // x flux with u's faces, rows i-2 .. i+1
+                const double* m = fb + (F == 1 ? RF_UY : RF_UZ) + uat;
+                const double2 t = flux<ORDER>(ORDER == 4 ? ld2(m - 2 * RT_J) : z2, ld2(m - RT_J), ld2(m),
+                                              ORDER == 4 ? ld2(m + RT_J) : z2, X(-3), X(-1), q0, X(1), X(3));
+                other = F == 1 ? t : other + t;
+            }
+            // z fluxes
+            double2 zph, zmh = f1, zp3 = z2, zm3 = ORDER == 4 ? ld2(f3q + ((k - 3) & 3) * 2 * RT_THREADS) : z2, mup;   // mup: m(k) at order 2, m(k+1) at order 4
+            if (F == 2) mup = ORDER == 2 ? 0.25 * (q0 + Z(1)) : face<ORDER>(q0, Z(1), Z(2), Z(NZ));
+            else mup = ld2(fb + (F == 0 ? RF_WX : RF_WY) + wat);
+            if (ORDER == 2) {
+                zph = mup * (q0 + Z(1));
+                f1 = zph;
+            } else {
+                zph = mz * (q0 + Z(1));
+                zp3 = mup * (q0 + Z(NZ));
+                f1 = zph;
+                st2(f3q + (k & 3) * 2 * RT_THREADS, zp3);
+                if (WALL && F < 2) {   // wall closures of the cell-centred fields: the wall value qbot / qtop
+                    auto wallq = [&](double2 a, double2 b, double2 c, double2 d) {   // ghost 2, ghost 1, first, second
+                        return (0.5 * A2) * (a + d) + (0.5 * (A1 + 2.0 * A2)) * (b + c);
+                    };
+                    if (k == top) {
+                        const double2 qt = wallq(Z(2), Z(1), q0, Z(-1));
+                        zph = (2.0 * mz) * qt;
+                        zp3 = (4.0 * mz) * qt - wface(k - 1) * (Z(-2) + Z(1));
+                    }
+                    if (k == top - 1) zp3 = (2.0 * mup) * wallq(Z(NZ), Z(2), Z(1), q0);
+                    if (k == GZ) {
+                        const double2 qb = wallq(Z(-2), Z(-1), q0, Z(1)), mb = wface(k - 1);
+                        zmh = (2.0 * mb) * qb;
+                        zm3 = (4.0 * mb) * qb - mz * (Z(2) + Z(-1));
+                    }
+                    if (k == GZ + 1) zm3 = (2.0 * wface(k - 2)) * wallq(Z(-NZ), Z(-2), Z(-1), q0);
+                }
+                mz = mup;
+            }
+            const double2 zs = ORDER == 2 ? dxdy * (zph - zmh) : dxdy * (A1 * (zph - zmh) + A2 * (zp3 - zm3));
+            if (F == 0) f = (-mrow[8]) * ((DYDZ(0) * own + DXDZ(0) * other) + zs);
+            if (F == 1) f = (-mrow[8]) * ((DYDZ(0) * other + DXDZ(0) * own) + zs);
+            if (F == 2) f = (-mrow[9]) * (other + zs);
+            // add_buoyancy{2,4} (scalar.c:6-76); skipped when every betg is zero
+            if (buoyancy) {
+                const double* c = ringat(3, k);
+                const double2 c0 = ld2(c);
+                if (F == 0) {
+                    const double2 t = ORDER == 2 ? 0.5 * (c0 + ld2(c + PJ))
+                                                 : B1 * (c0 + ld2(c + PJ)) + B2 * (ld2(c - PJ) + ld2(c + 2 * PJ));
+                    f = f + A.betg_x * t;
+                } else if (F == 1) {
+                    const double2 a = ld2(c - 2), b = ld2(c + 2), n = make_double2(c0.y, b.x);
+                    const double2 t = ORDER == 2 ? 0.5 * (c0 + n) : B1 * (c0 + n) + B2 * (make_double2(a.y, c0.x) + b);
+                    f = f + A.betg_y * t;
+                } else {
+                    const double2 n = ld2(ringat(3, k + 1));
+                    const double2 t = ORDER == 2 ? 0.5 * (c0 + n)
+                                                 : B1 * (c0 + n) + B2 * (ld2(ringat(3, k - 1)) + ld2(ringat(3, k + 2)));
+                    f = f + A.betg_z * t;
+                }
+            }
+        }
+        if (MODE != RHS_CHANNEL) f = f + lap;
+
+        // ---- right-hand side of the implicit solve, rows GZ .. (u, v, c: nz rows; w: nz - 1 faces)
+        const double2* r2 = reinterpret_cast<const double2*>(cst + (k & 1) * RT_FWMAX);
         double r[RT_FWMAX];
 #pragma unroll
-        for (int q = 0; q < (FWR + 1) / 2; q++) {
-            const double2 t = r2[q];
-            r[2 * q] = t.x;
-            r[2 * q + 1] = t.y;
+        for (int e = 0; e < (FWR + 1) / 2; e++) {
+            if (2 * e < 2 * HH + 4 || MODE == RHS_SWEEP) {
+                const double2 t = r2[e];
+                r[2 * e] = t.x;
+                r[2 * e + 1] = t.y;
+            }
         }
-        double sk = r[2 * H + 3] + r[2 * H + 1] * fk + r[2 * H + 2] * gk;
-#pragma unroll
-        for (int q = 0; q < 2 * H + 1; q++) sk += r[q] * X(q - H);
-        if (MODE == RHS_CHANNEL) return sk + lk;
-        if (MODE == RHS_H) return sk;
-        if (ORDER == 4) sk -= r[2 * H + 5] * s2 + r[2 * H + 6] * s3;
-        sk -= r[2 * H + 4] * s1;   // the previous row's s enters last
-        s3 = s2; s2 = s1; s1 = sk;
-        return sk;
-    };
-
-    // One row.  WALL: rows within two of a wall, whose z fluxes use the wall
-    // closures (and the top row has no w point), and the row whose w-solve
-    // window reaches above the top face; other rows take a branch-free path.
-    auto row = [&](auto wall_tag) {
-        constexpr bool WALL = decltype(wall_tag)::value;
-        const double ivol = mst[(k & 1) * RT_MROW + 8], ivolw = mst[(k & 1) * RT_MROW + 9];
-        const bool do_w = !WALL || k < n2 - GZ - 1;
-        const long long ijk = (long long) k * plane + gij;
-        const double* gk = gst + (k & 1) * 4 * RT_THREADS + tid;   // g of this row (staged)
-        const double gu = gk[0] + shift_u, gv = gk[RT_THREADS];
-        const double gw = gk[2 * RT_THREADS], gc = gk[3 * RT_THREADS] + shift_c;
-        double fu, fv, fw = 0.0, fc;
-        double lu, lv, lw = 0.0, lc;   // x-y diffusion terms
-
-        if (ORDER == 2) {
-            auto adv_cell = [&](auto Q, auto MX, auto MY, auto MZ) {   // advectu2 / advectv2 (advect.c:286-417)
-                double q0 = Q(0, 0, 0);
-                double xph = MX(0, 0, 0) * 0.5 * (q0 + Q(1, 0, 0));
-                double yph = MY(0, 0, 0) * 0.5 * (q0 + Q(0, 1, 0));
-                double zph = MZ(0, 0, 0) * 0.5 * (q0 + Q(0, 0, 1));
-                double xmh = MX(-1, 0, 0) * 0.5 * (q0 + Q(-1, 0, 0));
-                double ymh = MY(0, -1, 0) * 0.5 * (q0 + Q(0, -1, 0));
-                double zmh = MZ(0, 0, -1) * 0.5 * (q0 + Q(0, 0, -1));
-                if (WALL) {
-                    if (k == n2 - GZ - 1) zph = MZ(0, 0, 0) * (0.5 * (Q(0, 0, kt_u - 1 - k) + Q(0, 0, kt_u - k)));
-                    if (k == GZ) zmh = MZ(0, 0, -1) * (0.5 * (Q(0, 0, kb_w - k) + Q(0, 0, kb_w + 1 - k)));
-                }
-                return -((xph - xmh) + (yph - ymh) + (zph - zmh)) * ivol;
-            };
-            fu = adv_cell(U, mx_u2, mx_v2, mx_w2);
-            fv = adv_cell(V, my_u2, my_v2, my_w2);
-            if (do_w) {   // advectw2 (advect.c:420-463)
-                double q0 = W(0, 0, 0);
-                double xph = mz_u2(0, 0, 0) * 0.5 * (q0 + W(1, 0, 0));
-                double yph = mz_v2(0, 0, 0) * 0.5 * (q0 + W(0, 1, 0));
-                double zph = mz_w2(0, 0, 0) * 0.5 * (q0 + W(0, 0, 1));
-                double xmh = mz_u2(-1, 0, 0) * 0.5 * (q0 + W(-1, 0, 0));
-                double ymh = mz_v2(0, -1, 0) * 0.5 * (q0 + W(0, -1, 0));
-                double zmh = mz_w2(0, 0, -1) * 0.5 * (q0 + W(0, 0, -1));
-                fw = -((xph - xmh) + (yph - ymh) + (zph - zmh)) * ivolw;
-            }
-            // add_laplacexy_operator_{u,w}2 (diffuseu.c:286-313, diffusew.c:290-317)
-            auto lap2 = [&](auto F, double nu) {
-                double q0 = F(0, 0, 0);
-                return nu * (((F(1, 0, 0) - q0) * idx - (q0 - F(-1, 0, 0)) * idx) * idx
-                             + ((F(0, 1, 0) - q0) * idy - (q0 - F(0, -1, 0)) * idy) * idy);
-            };
-            lu = lap2(U, A.nu);
-            lv = lap2(V, A.nu);
-            if (do_w) lw = lap2(W, A.nu);
-            lc = lap2(C, A.kappa);
-        } else {
-            // advectu4 / advectv4 / advectw4 (advect.c:466-734).  Within one
-            // cell every x-direction mass flux carries the same metric
-            // (dydz[k] for the u-flux, dxdz[k] for the v-flux), so it is
-            // factored out of the x and y flux sums; the halved interpolation
-            // weights B1h, B2h absorb the 0.5 of the face value (an exact
-            // scaling).  Mathematically the reference's sums; they round
-            // differently.  The wall-adjacent z fluxes use the fourth-order
-            // wall value qbot / qtop; the z fluxes come from the per-field
-            // queue (zph / zp3 of this row, zmh / zm3 = zph of row k-1 / zp3
-            // of row k-3).
-            auto ix = [&](auto F, int di, int dj) {   // x interpolation to the face i+di+1/2
-                return B1h * (F(di, dj, 0) + F(di + 1, dj, 0)) + B2h * (F(di - 1, dj, 0) + F(di + 2, dj, 0));
-            };
-            auto iy = [&](auto F, int di, int dj) {   // y interpolation to the face j+dj+1/2
-                return B1h * (F(di, dj, 0) + F(di, dj + 1, 0)) + B2h * (F(di, dj - 1, 0) + F(di, dj + 2, 0));
-            };
-            auto xflux = [&](auto Q, auto M, double q0) {   // A1 (xph - xmh) + A2 (xp3 - xm3), metric factored out
-                return A1 * (M(0, 0) * (q0 + Q(1, 0, 0)) - M(-1, 0) * (q0 + Q(-1, 0, 0)))
-                     + A2 * (M(1, 0) * (q0 + Q(3, 0, 0)) - M(-2, 0) * (q0 + Q(-3, 0, 0)));
-            };
-            auto yflux = [&](auto Q, auto M, double q0) {
-                return A1 * (M(0, 0) * (q0 + Q(0, 1, 0)) - M(0, -1) * (q0 + Q(0, -1, 0)))
-                     + A2 * (M(0, 1) * (q0 + Q(0, 3, 0)) - M(0, -2) * (q0 + Q(0, -3, 0)));
-            };
-            auto zsum = [&](auto Q, auto MZ, double zph, double zmh, double zp3, double zm3) {
-                if (WALL) {
-                    double qbot = 0.5 * A2 * (Q(0, 0, kb_w - 1 - k) + Q(0, 0, kb_w + 2 - k))
-                                + 0.5 * (A1 + 2.0 * A2) * (Q(0, 0, kb_w - k) + Q(0, 0, kb_w + 1 - k));
-                    double qtop = 0.5 * A2 * (Q(0, 0, kt_u - 2 - k) + Q(0, 0, kt_u + 1 - k))
-                                + 0.5 * (A1 + 2.0 * A2) * (Q(0, 0, kt_u - 1 - k) + Q(0, 0, kt_u - k));
-                    if (k == n2 - GZ - 1) {
-                        zph = MZ(0, 0, 0) * qtop;
-                        zp3 = -MZ(0, 0, -1) * 0.5 * (Q(0, 0, -2) + Q(0, 0, 1)) + 2.0 * MZ(0, 0, 0) * qtop;
-                    }
-                    if (k == n2 - GZ - 2) zp3 = MZ(0, 0, 1) * qtop;
-                    if (k == GZ) {
-                        zmh = MZ(0, 0, -1) * qbot;
-                        zm3 = -MZ(0, 0, 0) * 0.5 * (Q(0, 0, 2) + Q(0, 0, -1)) + 2.0 * MZ(0, 0, -1) * qbot;
-                    }
-                    if (k == GZ + 1) zm3 = MZ(0, 0, -2) * qbot;
-                }
-                return A1 * (zph - zmh) + A2 * (zp3 - zm3);
-            };
-            const double mdy = DYDZ(0), mdx = DXDZ(0);
-            zq_u.advance(U, mx_w);
-            zq_v.advance(V, my_w);
-            {
-                const double q0 = U(0, 0, 0);
-                auto mu = [&](int di, int dj) { return ix(U, di, dj); };
-                auto mv = [&](int di, int dj) { return ix(V, di, dj); };
-                fu = -((mdy * xflux(U, mu, q0) + mdx * yflux(U, mv, q0))
-                       + zsum(U, mx_w, zq_u.f1, zq_u.f1m, zq_u.f3, zq_u.f3m[0])) * ivol;
-            }
-            {
-                const double q0 = V(0, 0, 0);
-                auto mu = [&](int di, int dj) { return iy(U, di, dj); };
-                auto mv = [&](int di, int dj) { return iy(V, di, dj); };
-                fv = -((mdy * xflux(V, mu, q0) + mdx * yflux(V, mv, q0))
-                       + zsum(V, my_w, zq_v.f1, zq_v.f1m, zq_v.f3, zq_v.f3m[0])) * ivol;
-            }
-            if (do_w) {
-                zq_w.advance(W, mz_w);
-                // z interpolation of the u / v mass fluxes to the w face: the
-                // metric differs per plane, folded into four row constants
-                const double cu0 = B1h * DYDZ(0), cu1 = B1h * DYDZ(1), cum = B2h * DYDZ(-1), cu2 = B2h * DYDZ(2);
-                const double cv0 = B1h * DXDZ(0), cv1 = B1h * DXDZ(1), cvm = B2h * DXDZ(-1), cv2 = B2h * DXDZ(2);
-                auto mu = [&](int di, int dj) {
-                    return (cu0 * U(di, dj, 0) + cu1 * U(di, dj, 1)) + (cum * U(di, dj, -1) + cu2 * U(di, dj, 2));
-                };
-                auto mv = [&](int di, int dj) {
-                    return (cv0 * V(di, dj, 0) + cv1 * V(di, dj, 1)) + (cvm * V(di, dj, -1) + cv2 * V(di, dj, 2));
-                };
-                const double q0 = W(0, 0, 0);
-                fw = -((xflux(W, mu, q0) + yflux(W, mv, q0))
-                       + (A1 * (zq_w.f1 - zq_w.f1m) + A2 * (zq_w.f3 - zq_w.f3m[0]))) * ivolw;
-            }
-            // add_laplacexy_operator_{u,w}4 (diffuseu.c:316-359, diffusew.c:320-363):
-            // A1 (d+1/2 - d-1/2) + A2 (d+3/2 - d-3/2) of the staggered first
-            // differences is the 7-point stencil L1, L2, L3, here in sum form:
-            // the symmetric pairs, then the centre weight -2 (L1 + L2 + L3)
-            // folded with both directions (lapc).  Mathematically the same;
-            // it rounds differently (the centre term no longer cancels
-            // exactly, an error of a few ulps of |u| (1/dx^2 + 1/dy^2) nu).
-            auto lap4 = [&](auto F, double nu) {
-                const double lx = L3 * (F(3, 0, 0) + F(-3, 0, 0)) + L2 * (F(2, 0, 0) + F(-2, 0, 0))
-                                + L1 * (F(1, 0, 0) + F(-1, 0, 0));
-                const double ly = L3 * (F(0, 3, 0) + F(0, -3, 0)) + L2 * (F(0, 2, 0) + F(0, -2, 0))
-                                + L1 * (F(0, 1, 0) + F(0, -1, 0));
-                return nu * ((lx * idx2 + ly * idy2) + lapc * F(0, 0, 0));
-            };
-            lu = lap4(U, A.nu);
-            lv = lap4(V, A.nu);
-            if (do_w) lw = lap4(W, A.nu);
-            lc = lap4(C, A.kappa);
-        }
-        if (MODE != RHS_CHANNEL) {
-            fu += lu;
-            fv += lv;
-            fw += lw;
-        }
-        fc = MODE == RHS_CHANNEL ? 0.0 : lc;
-
-        {   // flux_quick + advect_scalar (scalar.c:79-162), order independent
-            const double c0 = C(0, 0, 0);
-            const double kx0 = curv(C(1, 0, 0), c0, C(-1, 0, 0)), ky0 = curv(C(0, 1, 0), c0, C(0, -1, 0));
-            const double kxm = curv(c0, C(-1, 0, 0), C(-2, 0, 0)), kxp = curv(C(2, 0, 0), C(1, 0, 0), c0);
-            const double kym = curv(c0, C(0, -1, 0), C(0, -2, 0)), kyp = curv(C(0, 2, 0), C(0, 1, 0), c0);
-            const double kzp = curv(C(0, 0, 2), C(0, 0, 1), c0);
-            double fxp = quick(DYDZ(0) * U(0, 0, 0), c0, C(1, 0, 0), kx0, kxp);
-            double fxm = quick(DYDZ(0) * U(-1, 0, 0), C(-1, 0, 0), c0, kxm, kx0);
-            double fyp = quick(DXDZ(0) * V(0, 0, 0), c0, C(0, 1, 0), ky0, kyp);
-            double fym = quick(DXDZ(0) * V(0, -1, 0), C(0, -1, 0), c0, kym, ky0);
-            double fzp = quick(dxdy * W(0, 0, 0), c0, C(0, 0, 1), kz, kzp);
-            kz = kzp;
-            double fzm = fzp_prev;   // the top-face flux of row k-1
-            fzp_prev = fzp;
-            fc = -((fxp - fxm) + (fyp - fym) + (fzp - fzm)) * ivol + fc;
-            // add_buoyancy{2,4} (scalar.c:6-76)
-            if (!buoyancy) {
-            } else if (ORDER == 2) {
-                fu += 0.5 * (c0 + C(1, 0, 0)) * A.betg_x;
-                fv += 0.5 * (c0 + C(0, 1, 0)) * A.betg_y;
-                if (do_w) fw += 0.5 * (c0 + C(0, 0, 1)) * A.betg_z;
+        double2 h = r[2 * HH + 1] * f + r[2 * HH + 2] * gk;
+        h.x += r[2 * HH + 3];
+        h.y += r[2 * HH + 3];
+        // the old w beyond its wall faces is apply_bc_w's (the ring holds the massflux4 extrapolation)
+        double2 b1 = z2, b2 = z2;
+        if (WALL && F == 2 && ORDER == 4) {
+            double u;
+            if (k <= GZ + 1) {
+                const double2 w0 = k == GZ ? q0 : Z(-1), w1 = k == GZ ? Z(1) : q0;
+                bc_w_bot<4>(A.wbot, A.wbc_bot, w0.x, w1.x, u, b1.x, b2.x);
+                bc_w_bot<4>(A.wbot, A.wbc_bot, w0.y, w1.y, u, b1.y, b2.y);
             } else {
-                double cphx = B1 * (c0 + C(1, 0, 0)) + B2 * (C(-1, 0, 0) + C(2, 0, 0));
-                double cphy = B1 * (c0 + C(0, 1, 0)) + B2 * (C(0, -1, 0) + C(0, 2, 0));
-                fu += cphx * A.betg_x;
-                fv += cphy * A.betg_y;
-                if (do_w) fw += (B1 * (c0 + C(0, 0, 1)) + B2 * (C(0, 0, -1) + C(0, 0, 2))) * A.betg_z;
+                const double2 w0 = k == top - 2 ? Z(1) : q0, w1 = k == top - 2 ? q0 : Z(-1);
+                bc_w_top<4>(A.wtop, A.wbc_top, w0.x, w1.x, u, b1.x, b2.x);
+                bc_w_top<4>(A.wtop, A.wbc_top, w0.y, w1.y, u, b1.y, b2.y);
             }
         }
-
-        // forward sweeps of the implicit solves, rows k0 = GZ .. (u, v, c: nz
-        // rows; w: nz - 1 faces)
-        if (WALL && k >= n2 - GZ - 3)   // old w above the top face (apply_bc_w)
-            bc_w_top<ORDER>(A.wtop, A.wbc_top, W(0, 0, n2 - GZ - 2 - k), W(0, 0, n2 - GZ - 3 - k), gt0, gt1, gt2);
-        auto XW = [&](int dk) -> double {
-            if (WALL) {
-                const int kk = k + dk;
-                if (kk < GZ - 1) return kk == GZ - 2 ? gb1 : gb2;
-                if (kk > n2 - GZ - 1) return kk == n2 - GZ ? gt1 : gt2;
+#pragma unroll
+        for (int d = -HH; d <= HH; d++) {
+            double2 v = Z(d);
+            if (WALL && F == 2 && ORDER == 4) {
+                const int kk = k + d;
+                if (kk < GZ - 1) v = kk == GZ - 2 ? b1 : b2;
+                if (kk > top) v = kk == top + 1 ? b1 : b2;
             }
-            return W(0, 0, dk);
-        };
-        (void) gt0;
-        const double s_u = sweep(0, [&](int dk) { return U(0, 0, dk); }, fu, gu, lu, su1, su2, su3);
-        const double s_v = sweep(1, [&](int dk) { return V(0, 0, dk); }, fv, gv, lv, sv1, sv2, sv3);
-        const double s_w = do_w ? sweep(2, XW, fw, gw, lw, sw1, sw2, sw3) : 0.0;
-        const double s_c = sweep(3, [&](int dk) { return C(0, 0, dk); }, fc, gc, lc, sc1, sc2, sc3);
-        if (out) {
-            A.fu[ijk] = fu;
-            A.fv[ijk] = fv;
-            A.fc[ijk] = fc;
-            A.sw[0].g[ijk] = s_u;
-            A.sw[1].g[ijk] = s_v;
-            A.sw[3].g[ijk] = s_c;
-            if (do_w) {
-                A.fw[ijk] = fw;
-                A.sw[2].g[ijk] = s_w;
+            h = h + r[d + HH] * v;
+        }
+        if (MODE == RHS_CHANNEL) h = h + lap;
+        if (MODE == RHS_SWEEP) {
+            if (ORDER == 4) {
+                h = (h - r[2 * HH + 6] * s3) - r[2 * HH + 5] * s2;
+                s3 = s2;
+                s2 = s1;
+            }
+            h = h - r[2 * HH + 4] * s1;   // the previous row's s enters last
+            s1 = h;
+        }
+        if (live) {
+            if (EVEN) {
+                if (T.v0) {
+                    st2(fout, f);
+                    st2(gio, h);
+                }
+            } else {
+                if (T.v0) { fout[0] = f.x; gio[0] = h.x; }
+                if (T.v1) { fout[1] = f.y; gio[1] = h.y; }
             }
         }
+        fout += T.plane;
+        gio += T.plane;
     };
 
-    for (; k < ke; k++) {
-        if (k + 1 < ke) load_extras(k + 1);
-        if (k + T::ZH + 1 <= ke + T::ZH - 1) load_plane(k + T::ZH + 1);   // the last row reads ke - 1 + ZH
-        else cp_async_commit();
-        if (k <= GZ + 1 || k >= n2 - GZ - 3) row(std::true_type{});
-        else row(std::false_type{});
+    auto begin = [&](int k) {
+        if (k + 1 < T.ke) {
+            load_extras(k + 1);
+            load_plane(k + RT::ZH + 1);   // row k + 1 reads up to k + 1 + ZH
+        }
+    };
+    auto end = [&]() {
+        // This field's threads alone: a field reads its own newest plane and its
+        // own coefficients; of the others' planes rows up to k + 2 (order 2: k + 1),
+        // which landed a row or more before the last block-wide barrier.  That
+        // barrier also keeps a field within one row of the others: a ring slot
+        // or a face buffer is rewritten only after every reader has passed it.
         cp_async_wait_all();
-        __syncthreads();
+        asm volatile("bar.sync %0, %1;\n" ::"n"(F + 1), "n"(RT_FIELD) : "memory");
+    };
+    for (int k = T.kb; k < T.ke;) {
+        const int inner = min(T.ke, top - 2);
+        if (k > GZ + 1 && k < inner) {
+            for (; k < inner; k++) {
+                begin(k);
+                row(k, std::false_type{});
+                end();
+            }
+        } else {
+            begin(k);
+            row(k, std::true_type{});
+            end();
+            k++;
+        }
     }
 }
 
-template <int ORDER, int MODE>
-__global__ void __launch_bounds__(RT_THREADS, RhsTile<ORDER>::BLOCKS) k_rhs(Geo G, RhsArgs A)
+template <int ORDER, int MODE, bool EVEN>
+__device__ __forceinline__ void rhs_body(const Geo& G, const RhsArgs& A, uint3 bid)
 {
-    rhs_body<ORDER, MODE>(G, A, blockIdx);
+    using RT = RhsTile<ORDER>;
+    RhsBlock T;
+    int* goff = reinterpret_cast<int*>(rhs_sm + rhs_offs<ORDER>());
+    const int nx = G.nx, ny = G.ny, tid = threadIdx.x;
+    T.i0 = bid.y * RT_I;
+    T.j0 = bid.x * RT_J;
+    T.kb = GZ + (int) bid.z * A.chunk;
+    T.ke = min(T.kb + A.chunk, GZ + G.nz);
+    T.q = (tid >> 7) * 32 + (tid & 31);
+    T.ty = T.q >> 4;
+    T.jl = 2 * (T.q & 15);
+    T.plane = G.plane;
+    const int i = T.i0 + T.ty, j = T.j0 + T.jl;
+    T.v0 = i < nx && j < ny;
+    T.v1 = i < nx && j + 1 < ny;
+    T.gij = T.v0 ? (long long) i * ny + j : 0;
+    // The points (even ny: pairs) of a haloed plane, the same in every plane and
+    // field: their offsets within a plane.  For even ny a pair starts at an
+    // even y index (j0 and XL are even), so it never straddles the periodic
+    // wrap and its global and shared addresses are 16-byte aligned.
+    for (int e = tid; e < (EVEN ? RT::PLANE / 2 : RT::PLANE); e += RT_THREADS) {
+        const int w = EVEN ? RT::PJ / 2 : RT::PJ, ii = e / w, jj = (e - ii * w) * (EVEN ? 2 : 1);
+        int gi = (T.i0 + ii - RT::H) % nx; if (gi < 0) gi += nx;
+        int gj = (T.j0 + jj - RT::XL) % ny; if (gj < 0) gj += ny;
+        goff[e] = gi * ny + gj;
+    }
+    __syncthreads();
+    // Warp w works on field w mod 4, so that the warps of one of the SM's four
+    // schedulers run the same code.  Every field takes the same barriers.
+    switch ((tid >> 5) & 3) {
+    case 0: rhs_field<ORDER, MODE, 0, EVEN>(G, A, T); break;
+    case 1: rhs_field<ORDER, MODE, 1, EVEN>(G, A, T); break;
+    case 2: rhs_field<ORDER, MODE, 2, EVEN>(G, A, T); break;
+    default: rhs_field<ORDER, MODE, 3, EVEN>(G, A, T); break;
+    }
 }
 
-template <int ORDER>
-__global__ void __launch_bounds__(RT_THREADS, RhsTile<ORDER>::BLOCKS) k_rhs_batch(const BatchRec<RhsArgs>* r, int n)
+template <int ORDER, int MODE, bool EVEN>
+__global__ void __launch_bounds__(RT_THREADS, 1) k_rhs(Geo G, RhsArgs A)
+{
+    rhs_body<ORDER, MODE, EVEN>(G, A, blockIdx);
+}
+
+template <int ORDER, bool EVEN>
+__global__ void __launch_bounds__(RT_THREADS, 1) k_rhs_batch(const BatchRec<RhsArgs>* r, int n)
 {
     uint3 b;
     const BatchRec<RhsArgs>& R = batch_locate(r, n, b);
-    rhs_body<ORDER, RHS_SWEEP>(R.G, R.A, b);
+    rhs_body<ORDER, RHS_SWEEP, EVEN>(R.G, R.A, b);
 }
 
 // ------------------------------------------------------------- launchers
@@ -693,20 +761,28 @@ void launch_ghosts_batch(const BatchLaunch& L, int order, cudaStream_t st)
     else k_ghosts_batch<4, true><<<L.blocks, GHOST_THREADS, 0, st>>>(r, L.n);
 }
 
-// (whole columns in a batch: line_partitioned)
-void launch_rhs_batch(const BatchLaunch& L, int order, cudaStream_t st)
+// (whole columns in a batch: line_partitioned; key: order, + 8 for odd ny)
+void launch_rhs_batch(const BatchLaunch& L, int key, cudaStream_t st)
 {
     auto r = static_cast<const BatchRec<RhsArgs>*>(L.recs);
-    const dim3 blk(RT_J, RT_I, 1);
-    if (order == 2) k_rhs_batch<2><<<L.blocks, blk, rhs_smem_bytes<2>(), st>>>(r, L.n);
-    else k_rhs_batch<4><<<L.blocks, blk, rhs_smem_bytes<4>(), st>>>(r, L.n);
+    const dim3 blk(RT_THREADS);
+    switch (key) {
+    case 2: k_rhs_batch<2, true><<<L.blocks, blk, rhs_smem_bytes<2>(), st>>>(r, L.n); break;
+    case 4: k_rhs_batch<4, true><<<L.blocks, blk, rhs_smem_bytes<4>(), st>>>(r, L.n); break;
+    case 10: k_rhs_batch<2, false><<<L.blocks, blk, rhs_smem_bytes<2>(), st>>>(r, L.n); break;
+    default: k_rhs_batch<4, false><<<L.blocks, blk, rhs_smem_bytes<4>(), st>>>(r, L.n); break;
+    }
 }
 
 void launch_rhs(const Geo& G, const RhsArgs& A, bool implicit3d, cudaStream_t st)
 {
-    const dim3 blk(RT_J, RT_I, 1), grd = grid_rhs(G, A.chunk);
+    const dim3 blk(RT_THREADS), grd = grid_rhs(G, A.chunk);
     const int mode = implicit3d ? RHS_CHANNEL : G.partitioned ? RHS_H : RHS_SWEEP;
-#define CASE_(o_, m_) if (G.order == o_ && mode == m_) k_rhs<o_, m_><<<grd, blk, rhs_smem_bytes<o_>(), st>>>(G, A);
+#define CASE_(o_, m_) \
+    if (G.order == o_ && mode == m_) { \
+        if (G.ny % 2 == 0) k_rhs<o_, m_, true><<<grd, blk, rhs_smem_bytes<o_>(), st>>>(G, A); \
+        else k_rhs<o_, m_, false><<<grd, blk, rhs_smem_bytes<o_>(), st>>>(G, A); \
+    }
     CASE_(2, RHS_SWEEP) CASE_(2, RHS_H) CASE_(2, RHS_CHANNEL)
     CASE_(4, RHS_SWEEP) CASE_(4, RHS_H) CASE_(4, RHS_CHANNEL)
 #undef CASE_
@@ -719,14 +795,22 @@ cudaError_t rhs_set_smem_limits()
     auto set = [&](const void* f, int v) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
     };
-    set((const void*) k_rhs<2, RHS_SWEEP>, v2);
-    set((const void*) k_rhs<2, RHS_H>, v2);
-    set((const void*) k_rhs<2, RHS_CHANNEL>, v2);
-    set((const void*) k_rhs<4, RHS_SWEEP>, v4);
-    set((const void*) k_rhs<4, RHS_H>, v4);
-    set((const void*) k_rhs<4, RHS_CHANNEL>, v4);
-    set((const void*) k_rhs_batch<2>, v2);
-    set((const void*) k_rhs_batch<4>, v4);
+    set((const void*) k_rhs<2, RHS_SWEEP, true>, v2);
+    set((const void*) k_rhs<2, RHS_SWEEP, false>, v2);
+    set((const void*) k_rhs<2, RHS_H, true>, v2);
+    set((const void*) k_rhs<2, RHS_H, false>, v2);
+    set((const void*) k_rhs<2, RHS_CHANNEL, true>, v2);
+    set((const void*) k_rhs<2, RHS_CHANNEL, false>, v2);
+    set((const void*) k_rhs<4, RHS_SWEEP, true>, v4);
+    set((const void*) k_rhs<4, RHS_SWEEP, false>, v4);
+    set((const void*) k_rhs<4, RHS_H, true>, v4);
+    set((const void*) k_rhs<4, RHS_H, false>, v4);
+    set((const void*) k_rhs<4, RHS_CHANNEL, true>, v4);
+    set((const void*) k_rhs<4, RHS_CHANNEL, false>, v4);
+    set((const void*) k_rhs_batch<2, true>, v2);
+    set((const void*) k_rhs_batch<2, false>, v2);
+    set((const void*) k_rhs_batch<4, true>, v4);
+    set((const void*) k_rhs_batch<4, false>, v4);
     return e;
 }
 
