@@ -6,7 +6,11 @@ and the packed x transforms change form, against the numpy restatement:
   column (192 rows) and the first whole-column one (193);
 * planes whose columns do not fill the last group of 16 (or of 32), odd and even;
 * x transforms of two columns each: an odd last column, 16-column blocks with
-  one column and with fifteen.
+  one column and with fifteen;
+* transforms planned at run time: one stage (4, 5), the largest size (500),
+  each radix first and last, lines that do not fill a block of 8;
+* the divergence's loads ahead: a plane's last positions that fill part of a
+  turn of 16, with fixed (48, 192, 320) and planned sizes.
 
 Bars as test_gpu_parity.py: relative L2 1e-13 on u, v, w, c and 1e-10 on p
 (rounding of u* by 1e-16 is divided by dt and passes the inverse Laplacian),
@@ -22,9 +26,11 @@ pytestmark = pytest.mark.gpu
 
 CASES = [(2, 12, 15, 4), (4, 10, 9, 6), (2, 16, 18, 15), (4, 15, 81, 16), (2, 9, 16, 17), (4, 8, 25, 17),
          (4, 12, 30, 32), (2, 15, 45, 33), (4, 20, 6, 49), (4, 6, 5, 192), (2, 6, 5, 193), (4, 8, 10, 193)]
+TRANSFORMS = [(2, 500, 4, 4), (4, 5, 500, 6), (2, 4, 486, 5), (4, 243, 8, 6), (2, 40, 24, 4), (4, 200, 250, 6),
+              (4, 48, 18, 7), (2, 192, 30, 5), (4, 192, 9, 6), (4, 320, 15, 6)]
 
 
-@pytest.mark.parametrize("order,nx,ny,nz", CASES)
+@pytest.mark.parametrize("order,nx,ny,nz", CASES + TRANSFORMS)
 def test_substeps_match_restatement(cf, gpu, order, nx, ny, nz):
     prm = cn.Params(order=order, nx=nx, ny=ny, nz=nz, lx=2 * np.pi, ly=np.pi, lz=2.0, dt=1e-3, nu=1.0 / 3000.0,
                     prandtl=0.71, setuframe=0.3, betg_x=0.1, betg_y=0.05, betg_z=0.02)

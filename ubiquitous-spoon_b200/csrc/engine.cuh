@@ -268,7 +268,7 @@ void launch_fftx_c2r(const Geo& G, const C2rArgs& A, int nrows, cudaStream_t st,
 void launch_poisson(const Geo& G, const PoissonArgs& A, cudaStream_t st);
 void launch_helmholtz_spectral(const Geo& G, const PoissonArgs& A, cudaStream_t st);
 void launch_project(const Geo& G, const ProjArgs& A, cudaStream_t st);
-cudaError_t fft_set_smem_limits(int max_n);
+cudaError_t fft_set_smem_limits();
 
 // ------------------------------------------------- batched launches (batch.cuh)
 struct BatchLaunch;
@@ -307,7 +307,6 @@ void launch_helmholtz_fft_batch(const BatchLaunch& L, int order, int ny, cudaStr
 void launch_c2r_batch(const BatchLaunch& L, int nx, cudaStream_t st);    // nx: power of two, else generic
 void launch_project_batch(const BatchLaunch& L, int order, cudaStream_t st);
 cudaError_t rhs_set_smem_limits();
-size_t fft_smem_bytes(int n);
 constexpr int FFT_MAX_N = 512;
 
 }  // namespace cf

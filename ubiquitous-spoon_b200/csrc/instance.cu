@@ -1837,7 +1837,7 @@ static int create_impl(const cf_config* cfg, void* stream, cf_instance* I)
     rc = plan(C.ny, I->py, I->twy);
     if (rc) return rc;
     I->c8 = std::cos(M_PI / 4.0);
-    CF_CUDA(fft_set_smem_limits(std::max(C.nx, C.ny)));
+    CF_CUDA(fft_set_smem_limits());
     CF_CUDA(rhs_set_smem_limits());
     I->bc_ub = to_dev(bc_rows_u(I->m, true));
     I->bc_ut = to_dev(bc_rows_u(I->m, false));

@@ -41,18 +41,11 @@ __device__ __forceinline__ double2 cmul_si(double2 a, int s)
 }
 
 struct FftCtx {
-    double2* buf;
-    int N, L;
-    bool line_major;      // element (pos, line) at buf[line*N + pos], else buf[pos*L + line]
+    int N;
     int sign;             // -1 forward, +1 backward
     const double2* tw;    // exp(-2 pi i m / N)
     double c8;            // cos(pi/4) from the host table
 };
-
-__device__ __forceinline__ int fidx(const FftCtx& F, int pos, int line)
-{
-    return F.line_major ? line * F.N + pos : pos * F.L + line;
-}
 
 __device__ __forceinline__ double2 twid(const FftCtx& F, int m)
 {
@@ -89,86 +82,97 @@ __device__ __forceinline__ void dft_small(double2* v, const FftCtx& F)
         v[1] = cadd(e[1], o1);   v[5] = csub(e[1], o1);
         v[2] = cadd(e[2], o2);   v[6] = csub(e[2], o2);
         v[3] = cadd(e[3], o3);   v[7] = csub(e[3], o3);
+    } else if (R == 3) {
+        const double2 w = __ldg(&F.tw[F.N / 3]);   // roots of unity from the host table: (cos, -sin)
+        const double h = -s * w.y;
+        const double2 t = cadd(v[1], v[2]), d = csub(v[1], v[2]);
+        const double2 m = make_double2(v[0].x + w.x * t.x, v[0].y + w.x * t.y), e = make_double2(-h * d.y, h * d.x);
+        v[0] = cadd(v[0], t);
+        v[1] = cadd(m, e);
+        v[2] = csub(m, e);
     } else {
-        // generic (3, 5): roots of unity from the host table
-        double2 out[R];
-        const int step = F.N / R;
-#pragma unroll
-        for (int q = 0; q < R; q++) {
-            double2 acc = v[0];
-#pragma unroll
-            for (int r = 1; r < R; r++) acc = cadd(acc, cmul(v[r], twid(F, ((r * q) % R) * step)));
-            out[q] = acc;
-        }
-#pragma unroll
-        for (int q = 0; q < R; q++) v[q] = out[q];
-    }
-}
-
-// One Stockham stage of radix R (Ns = product of the previous radices).
-template <int R, int MAXB>
-__device__ void fft_stage(const FftCtx& F, int Ns)
-{
-    const int NR = F.N / R;
-    const int nb = NR * F.L;
-    const int nthr = blockDim.x, tid = threadIdx.x;
-    double2 v[MAXB][R];
-    int jj[MAXB], ll[MAXB];
-#pragma unroll
-    for (int t = 0; t < MAXB; t++) {
-        int b = tid + t * nthr;
-        jj[t] = -1;
-        if (b < nb) {
-            int line, j;
-            if (F.line_major) { line = b / NR; j = b - line * NR; }
-            else { j = b / F.L; line = b - j * F.L; }
-            jj[t] = j;
-            ll[t] = line;
-            int k = j % Ns;
-            int tstep = F.N / (Ns * R);
-#pragma unroll
-            for (int r = 0; r < R; r++) {
-                double2 a = F.buf[fidx(F, j + r * NR, line)];
-                if (r > 0 && k > 0) a = cmul(a, twid(F, (r * k * tstep) % F.N));
-                v[t][r] = a;
-            }
-            dft_small<R>(v[t], F);
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int t = 0; t < MAXB; t++) {
-        if (jj[t] < 0) continue;
-        int j = jj[t], k = j % Ns;
-        int idxD = (j / Ns) * Ns * R + k;
-#pragma unroll
-        for (int r = 0; r < R; r++) F.buf[fidx(F, idxD + r * Ns, ll[t])] = v[t][r];
-    }
-    __syncthreads();
-}
-
-// Full transform; `plan` radices multiply to N.  MAXC bounds N*L/blockDim.
-template <int MAXC>
-__device__ void fft_run(const FftCtx& F, const FftPlan& plan)
-{
-    int Ns = 1;
-    for (int s = 0; s < plan.nstages; s++) {
-        int R = plan.radix[s];
-        switch (R) {
-        case 2: fft_stage<2, MAXC / 2>(F, Ns); break;
-        case 3: fft_stage<3, MAXC / 3 + 1>(F, Ns); break;
-        case 4: fft_stage<4, MAXC / 4>(F, Ns); break;
-        case 5: fft_stage<5, MAXC / 5 + 1>(F, Ns); break;
-        default: fft_stage<8, MAXC / 8>(F, Ns); break;
-        }
-        Ns *= R;
+        const double2 w = __ldg(&F.tw[F.N / 5]), z = __ldg(&F.tw[2 * (F.N / 5)]);
+        const double h = -s * w.y, g = -s * z.y;
+        const double2 t = cadd(v[1], v[4]), d = csub(v[1], v[4]), p = cadd(v[2], v[3]), q = csub(v[2], v[3]);
+        const double2 m = make_double2(v[0].x + w.x * t.x + z.x * p.x, v[0].y + w.x * t.y + z.x * p.y);
+        const double2 n = make_double2(v[0].x + z.x * t.x + w.x * p.x, v[0].y + z.x * t.y + w.x * p.y);
+        const double2 e = make_double2(-(h * d.y + g * q.y), h * d.x + g * q.x);
+        const double2 f = make_double2(-(g * d.y - h * q.y), g * d.x - h * q.x);
+        v[0] = cadd(v[0], cadd(t, p));
+        v[1] = cadd(m, e); v[4] = csub(m, e);
+        v[2] = cadd(n, f); v[3] = csub(n, f);
     }
 }
 
 constexpr int FFT_L = 8;        // transforms per block
 constexpr int FFT_J = 16;       // columns of an x-transform block, two per transform
 constexpr int FFT_THREADS = 256;
-constexpr int FFT_MAXC = 16;    // N * L / threads for N <= 512
+
+// Transforms of a size known only at run time: slot of element `pos` of line
+// `line`, line-major padded (y transforms) or position-major (x transforms).
+__host__ __device__ __forceinline__ int lm_pitch(int N) { return N + N / 8 + 1; }
+
+template <bool LM>
+__device__ __forceinline__ int rslot(int N, int pos, int line)
+{
+    return LM ? line * lm_pitch(N) + pos + (pos >> 3) : pos * FFT_L + line;
+}
+
+// a / n for 0 <= a < 8192, 1 <= n <= 512, inv = 1 / n: the quotient is off by
+// at most 3 * 2^-24 of itself, (a + 1/2) / n lies 1 / 2n or more from any integer
+__device__ __forceinline__ int quot(int a, float inv) { return (int) (((float) a + 0.5f) * inv); }
+
+// One Stockham stage of radix R (Ns = product of the previous radices), from
+// one buffer into the other: a butterfly's registers live only within its turn
+// of the loop.  In place, every butterfly of a thread was held across the
+// barrier (1.3 KB of spills), and indices were divided as integers.  us per launch, before and after, along y forward and along x inverse:
+// 90 x 75 x 53 24 -> 12, 17 -> 11; 240 x 250 x 64 119 -> 47, 91 -> 35;
+// 480 x 500 x 48 (both buffers 128 and 144 KB, one block per SM) 329 -> 146, 232 -> 164.
+template <int R, bool LM>
+__device__ __forceinline__ void fft_stage(const double2* __restrict__ src, double2* __restrict__ dst, const FftCtx& F,
+                                          int Ns)
+{
+    const int N = F.N, NR = N / R, nb = NR * FFT_L, tstep = NR / Ns;
+    const float inr = 1.0f / (float) NR, ins = 1.0f / (float) Ns;
+    for (int b = threadIdx.x; b < nb; b += FFT_THREADS) {
+        const int line = LM ? quot(b, inr) : b % FFT_L, j = LM ? b - line * NR : b / FFT_L;
+        const int q = quot(j, ins), k = j - q * Ns;
+        double2 v[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) v[r] = src[rslot<LM>(N, j + r * NR, line)];
+        if (k > 0) {
+#pragma unroll
+            for (int r = 1; r < R; r++) v[r] = cmul(v[r], twid(F, r * k * tstep));   // r k tstep < N
+        }
+        dft_small<R>(v, F);
+#pragma unroll
+        for (int r = 0; r < R; r++) dst[rslot<LM>(N, q * Ns * R + k + r * Ns, line)] = v[r];
+    }
+    __syncthreads();
+}
+
+// Full transform of FFT_L lines in a; `plan` radices multiply to N.  Returns
+// the buffer, a or b, that holds the result.
+template <bool LM>
+__device__ __forceinline__ double2* fft_run(double2* a, double2* b, const FftCtx& F, const FftPlan& plan)
+{
+    int Ns = 1;
+    for (int s = 0; s < plan.nstages; s++) {
+        const int R = plan.radix[s];
+        switch (R) {
+        case 2: fft_stage<2, LM>(a, b, F, Ns); break;
+        case 3: fft_stage<3, LM>(a, b, F, Ns); break;
+        case 4: fft_stage<4, LM>(a, b, F, Ns); break;
+        case 5: fft_stage<5, LM>(a, b, F, Ns); break;
+        default: fft_stage<8, LM>(a, b, F, Ns); break;
+        }
+        Ns *= R;
+        double2* const t = a;
+        a = b;
+        b = t;
+    }
+    return a;
+}
 
 // ---------------------------------------------- transforms of a fixed size
 //
@@ -296,8 +300,8 @@ static bool static_fft_size(int n)
 // Dynamic shared memory of the generic transforms of size n.
 size_t fft_generic_smem(int n, bool line_major)
 {
-    if (static_fft_size(n) && line_major) return (size_t) FFT_L * (n + n / 8 + 1) * sizeof(double2);
-    return (size_t) n * FFT_L * sizeof(double2);
+    const size_t one = (size_t) FFT_L * (line_major ? lm_pitch(n) : n) * sizeof(double2);
+    return static_fft_size(n) ? one : 2 * one;   // the runtime plan works from one buffer into another
 }
 
 // --------------------------------------------------------- divergence + x FFT
@@ -320,49 +324,70 @@ __device__ __forceinline__ void k_div_fftx_body(const Geo& G, const DivArgs& A, 
     const int k = GZ + A.kshift + bid.y;
     const int j0 = bid.x * FFT_J;
     const int nx = N ? N : G.nx, ny = G.ny, n2 = G.n2;
-    const double dx = G.dx, dy = G.dy, dzk = G.dz[k];
-    const double uc = A.mu ? A.gu[k] * (*A.mu) : 0.0;   // chanfast.c:516-519
-    const bool corr = A.mu != nullptr;
-    auto I = [&](int kk, int i, int j) { return ((long long) kk * nx + i) * ny + j; };
-    const int kb = GZ - 1, kt = n2 - GZ - 1;
-    for (int idx = threadIdx.x; idx < nx * FFT_J; idx += blockDim.x) {
-        int i = idx / FFT_J, jj = idx - i * FFT_J, j = j0 + jj;
-        double d = 0.0;
-        if (j < ny && A.src) {
-            d = __ldg(A.src + I(k, i, j));
-        } else if (j < ny) {
-            auto U = [&](int di) { double t = __ldg(A.u + I(k, wrapp(i + di, nx), j)); return corr ? t + uc : t; };
-            auto V = [&](int dj) { return __ldg(A.v + I(k, i, wrapp(j + dj, ny))); };
-            auto Wr = [&](int kk) { return __ldg(A.w + I(kk, i, j)); };
+    // A thread keeps its column and takes FFT_THREADS / FFT_J positions a turn,
+    // four turns' loads in flight; the loop runs over G.nx also where the size
+    // is fixed (with a constant trip count the loads of the turns did not
+    // overlap: 92 us at 192 x 192 x 128, order 2).  One turn at a time, with its
+    // tests and divisions, left every load's latency open: 83 us there, 47 now;
+    // order 4 113 -> 72; 480 x 500 x 48 order 2 (planned size) 683 -> 187.
+    const int jj = threadIdx.x % FFT_J, j = j0 + jj;
+    double* const d0 = sreal + jj;
+    const long long at = (long long) k * G.nx * ny + j;
+    constexpr int STEP = FFT_THREADS / FFT_J;
+    const int i0 = threadIdx.x / FFT_J, rows = G.nx;
+    if (j >= ny) {
+        for (int i = i0; i < rows; i += STEP) d0[i * FFT_J] = 0.0;
+    } else if (A.src) {
+        const double* const f = A.src + at;
+#pragma unroll 4
+        for (int i = i0; i < rows; i += STEP) d0[i * FFT_J] = __ldg(f + (long long) i * ny);
+    } else {
+        const double rdx = 1.0 / G.dx, rdy = 1.0 / G.dy, rdz = 1.0 / G.dz[k];
+        const double uc = A.mu ? A.gu[k] * (*A.mu) : 0.0;   // chanfast.c:516-519
+        const long long sxy = (long long) rows * ny;
+        const double *const u = A.u + at, *const v = A.v + at, *const w = A.w + at;
+        const int vm1 = wrapp(j - 1, ny) - j, vp1 = wrapp(j + 1, ny) - j, vm2 = wrapp(j - 2, ny) - j;
+        const bool bot = k == GZ, top = k == n2 - GZ - 1;
+#pragma unroll 4
+        for (int i = i0; i < rows; i += STEP) {
+            const long long o = (long long) i * ny;
+            auto U = [&](int di) { return __ldg(u + (long long) wrapp(i + di, rows) * ny) + uc; };
+            double d;
             if (ORDER == 2) {
-                d = (U(0) - U(-1)) / dx + (V(0) - V(-1)) / dy + (Wr(k) - Wr(k - 1)) / dzk;
+                d = (U(0) - U(-1)) * rdx + (__ldg(v + o) - __ldg(v + o + vm1)) * rdy + (__ldg(w + o) - __ldg(w + o - sxy)) * rdz;
             } else {
-                double wkm2 = (k - 2 == kb - 1) ? 2.0 * Wr(kb) - Wr(kb + 1) : Wr(k - 2);  // pressure.c:80-87
-                double wkp1 = (k + 1 == kt + 1) ? 2.0 * Wr(kt) - Wr(kt - 1) : Wr(k + 1);  // pressure.c:88-95
-                d = (A1 * (U(0) - U(-1)) + A2 * (U(1) - U(-2))) / dx
-                  + (A1 * (V(0) - V(-1)) + A2 * (V(1) - V(-2))) / dy
-                  + (A1 * (Wr(k) - Wr(k - 1)) + A2 * (wkp1 - wkm2)) / dzk;
+                const double w0 = __ldg(w + o), w1 = __ldg(w + o - sxy);
+                double wm = __ldg(w + o - 2 * sxy), wp = __ldg(w + o + sxy);
+                if (bot) wm = 2.0 * w1 - w0;   // pressure.c:80-87
+                if (top) wp = 2.0 * w0 - w1;   // pressure.c:88-95
+                d = (A1 * (U(0) - U(-1)) + A2 * (U(1) - U(-2))) * rdx
+                  + (A1 * (__ldg(v + o) - __ldg(v + o + vm1)) + A2 * (__ldg(v + o + vp1) - __ldg(v + o + vm2))) * rdy
+                  + (A1 * (w0 - w1) + A2 * (wp - wm)) * rdz;
             }
+            d0[i * FFT_J] = d;
         }
-        sreal[idx] = d;
     }
     __syncthreads();
-    FftCtx F{sbuf, nx, FFT_L, false, -1, A.px.tw, A.c8};
+    FftCtx F{nx, -1, A.px.tw, A.c8};
+    const double2* out = sbuf;
     if constexpr (N > 0) fft_static<N, false>(sbuf, F);
-    else fft_run<FFT_MAXC>(F, A.px);
+    else out = fft_run<false>(sbuf, sbuf + FFT_L * nx, F, A.px);
     const int nkx = G.nkx;
     const double scale = 0.5 / (double) nx;
     for (int idx = threadIdx.x; idx < nkx * FFT_J; idx += blockDim.x) {
         int kx = idx / FFT_J, jj = idx - kx * FFT_J, j = j0 + jj;
         if (j >= ny) continue;
-        const double2 z = sbuf[kx * FFT_L + jj / 2], c = sbuf[(kx ? nx - kx : 0) * FFT_L + jj / 2];
+        const double2 z = out[kx * FFT_L + jj / 2], c = out[(kx ? nx - kx : 0) * FFT_L + jj / 2];
         const double2 t = jj & 1 ? make_double2(z.y + c.y, c.x - z.x) : make_double2(z.x + c.x, z.y - c.y);
         A.spec[((long long) k * nkx + kx) * ny + j] = make_double2(t.x * scale, t.y * scale);
     }
 }
 
+// Blocks per SM: 4 up to 192 (64 registers; with 5 the loads in flight
+// do not fit, 47 -> 52 us at 192 x 192 x 128), 3 at 320 and 384 (60 -> 55 us at
+// 320 x 384 x 48), 2 where the size is planned (3: 69 -> 82 us at 300 x 384 x 48).
 template <int ORDER, int N>
-__global__ void __launch_bounds__(FFT_THREADS) k_div_fftx(Geo G, DivArgs A)
+__global__ void __launch_bounds__(FFT_THREADS, N == 0 ? 2 : N <= 192 ? 4 : 3) k_div_fftx(Geo G, DivArgs A)
 {
     k_div_fftx_body<ORDER, N>(G, A, blockIdx);
 }
@@ -387,25 +412,21 @@ __device__ __forceinline__ void k_ffty_body(const Geo& G, const FftyArgs& A, uin
     const int ny = N ? N : G.ny, nkx = G.nkx;
     const int nl = min(FFT_L, nkx - kx0);
     double2* base = A.spec + bid.z * A.fstride + ((long long) k * nkx + kx0) * ny;
+    const float iny = 1.0f / (float) ny;
     auto slot = [&](int idx) {   // idx = line * ny + pos
-        if constexpr (N > 0) {
-            const int line = idx / N, pos = idx - line * N;
-            return sslot<N, true>(pos, line);
-        } else {
-            return idx;
-        }
+        const int line = N ? idx / ny : quot(idx, iny), pos = idx - line * ny;
+        return N ? sslot<N ? N : 8, true>(pos, line) : rslot<true>(ny, pos, line);
     };
-    for (int idx = threadIdx.x; idx < FFT_L * ny; idx += blockDim.x) {
-        int line = idx / ny;
-        sbuf[slot(idx)] = line < nl ? base[idx] : make_double2(0.0, 0.0);
-    }
+    for (int idx = threadIdx.x; idx < FFT_L * ny; idx += FFT_THREADS)
+        sbuf[slot(idx)] = idx < nl * ny ? base[idx] : make_double2(0.0, 0.0);
     __syncthreads();
-    FftCtx F{sbuf, ny, FFT_L, true, A.sign, A.py.tw, A.c8};
+    FftCtx F{ny, A.sign, A.py.tw, A.c8};
+    const double2* out = sbuf;
     if constexpr (N > 0) fft_static<N, true>(sbuf, F);
-    else fft_run<FFT_MAXC>(F, A.py);
+    else out = fft_run<true>(sbuf, sbuf + FFT_L * lm_pitch(ny), F, A.py);
     const double scale = 1.0 / (double) ny;
-    for (int idx = threadIdx.x; idx < nl * ny; idx += blockDim.x) {
-        double2 t = sbuf[slot(idx)];
+    for (int idx = threadIdx.x; idx < nl * ny; idx += FFT_THREADS) {
+        double2 t = out[slot(idx)];
         if (A.sign < 0) { t.x *= scale; t.y *= scale; }
         base[idx] = t;
     }
@@ -434,7 +455,6 @@ template <int N>
 __device__ __forceinline__ void k_fftx_c2r_body(const Geo& G, const C2rArgs& A, uint3 bid)
 {
     extern __shared__ double2 sbuf[];
-    const double* const sreal = reinterpret_cast<const double*>(sbuf);
     const int k = A.kfirst + bid.y;
     const int j0 = bid.x * FFT_J;
     const int nx = N ? N : G.nx, ny = G.ny, nkx = G.nkx;
@@ -449,9 +469,11 @@ __device__ __forceinline__ void k_fftx_c2r_body(const Geo& G, const C2rArgs& A, 
         if (kx && 2 * kx != nx) sbuf[(nx - kx) * FFT_L + l] = make_double2(a.x + b.y, b.x - a.y);
     }
     __syncthreads();
-    FftCtx F{sbuf, nx, FFT_L, false, +1, A.px.tw, A.c8};
+    FftCtx F{nx, +1, A.px.tw, A.c8};
+    const double2* out = sbuf;
     if constexpr (N > 0) fft_static<N, false>(sbuf, F);
-    else fft_run<FFT_MAXC>(F, A.px);
+    else out = fft_run<false>(sbuf, sbuf + FFT_L * nx, F, A.px);
+    const double* const sreal = reinterpret_cast<const double*>(out);
     double* const pz = bid.z == 0 ? A.p[0] : bid.z == 1 ? A.p[1] : bid.z == 2 ? A.p[2] : A.p[3];
     for (int idx = threadIdx.x; idx < nx * FFT_J; idx += blockDim.x) {
         int i = idx / FFT_J, jj = idx - i * FFT_J, j = j0 + jj;
@@ -1961,8 +1983,6 @@ static bool pow2_kernel_size(int n) { return n == 64 || n == 128 || n == 256 || 
 
 // -------------------------------------------------------------- launchers
 
-size_t fft_smem_bytes(int n) { return (size_t) n * FFT_L * sizeof(double2); }
-
 void launch_div_fftx(const Geo& G, const DivArgs& A, cudaStream_t st)
 {
     switch (G.nx) {
@@ -1973,7 +1993,7 @@ void launch_div_fftx(const Geo& G, const DivArgs& A, cudaStream_t st)
     default: break;
     }
     dim3 grd((G.ny + FFT_J - 1) / FFT_J, G.nz);
-    size_t sm = fft_smem_bytes(G.nx);
+    size_t sm = fft_generic_smem(G.nx, false);
 #define CASE_(n_) \
     case n_: \
         if (G.order == 2) k_div_fftx<2, n_><<<grd, FFT_THREADS, sm, st>>>(G, A); \
@@ -2002,7 +2022,7 @@ void launch_fft2d_field(const Geo& G, const double* field, double2* spec, const 
         D.src = field;
         D.kshift = -GZ;
         dim3 grd((G.ny + FFT_J - 1) / FFT_J, G.n2);
-        const size_t sm = fft_smem_bytes(G.nx);
+        const size_t sm = fft_generic_smem(G.nx, false);
 #define CASE_(n_) \
     case n_: k_div_fftx<2, n_><<<grd, FFT_THREADS, sm, st>>>(G, D); break;
         switch (G.nx) {
@@ -2062,7 +2082,7 @@ void launch_fftx_c2r(const Geo& G, const C2rArgs& A, int nrows, cudaStream_t st,
     default: break;
     }
     dim3 grd((G.ny + FFT_J - 1) / FFT_J, nrows, nfields);
-    const size_t sm = fft_smem_bytes(G.nx);
+    const size_t sm = fft_generic_smem(G.nx, false);
 #define CASE_(n_) \
     case n_: k_fftx_c2r<n_><<<grd, FFT_THREADS, sm, st>>>(G, A); return;
     switch (G.nx) {
@@ -2289,17 +2309,15 @@ bool batch_pow2(int n) { return pow2_kernel_size(n); }
 
 int fft_kernel_key(int n) { return pow2_kernel_size(n) || static_fft_size(n) ? n : 0; }
 
-cudaError_t fft_set_smem_limits(int max_n)
+cudaError_t fft_set_smem_limits()
 {
-    size_t sm = fft_smem_bytes(max_n);
     cudaError_t e = p2_set_smem<64>();
     if (e == cudaSuccess) e = p2_set_smem<128>();
     if (e == cudaSuccess) e = p2_set_smem<256>();
     if (e == cudaSuccess) e = p2_set_smem<512>();
-    (void) sm;
-    // generic transforms (single and batched): room for the largest size
-    // handled by the runtime plan and for the padded fixed-size buffers
-    const int v = (int) std::max(fft_smem_bytes(FFT_MAX_N), fft_generic_smem(384, true));
+    // generic transforms (single and batched): room for the two padded buffers
+    // of the largest size that the runtime plan handles
+    const int v = (int) fft_generic_smem(FFT_MAX_N, true);
     auto set = [&](const void* f) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
     };
