@@ -216,7 +216,9 @@ int cf_z_coords(const cf_instance *inst, double *zp, double *zw);         /* get
  * in device memory: geometry, arguments, own grid).  Members may differ in
  * grid size, order and physical parameters; they must use
  * CF_SCHEME_CHANFAST and live on one device.  Each member's results are the
- * same, bit for bit, as stepping it alone with cf_step.
+ * same, bit for bit, whatever the other members are, and agree with stepping
+ * it alone with cf_step to rounding (a batch solves whole columns, where
+ * cf_step cuts the columns of a small plane into chunks).
  *
  * cf_batch_step: advance every member by nsub substeps on `stream` (NULL:
  * the first member's stream), recording the launches on the spot.  Ordered
@@ -246,11 +248,11 @@ int cf_batch_destroy(cf_batch *batch);
 
 /* ------------------------------------------------------------------------
  * Launch-shape autotuning.  Three kernels run with any of a few block shapes
- * and give the same results bit for bit: the line solves (columns per block,
- * or threads of a partitioned block's columns: 64, 128), the Poisson / spectral Helmholtz band solve (column
- * pairs per block: 64, 128) and the projection (block of j by i: 32x2, 32x4,
- * 32x8, 64x2).  cf_create times the candidates on the new instance (before
- * it holds state) and keeps the fastest; cf_batch_create does the same on
+ * and give the same results bit for bit: the line solves (columns per
+ * block: 64, 128; on a small plane, chunks of up to 96, 192 threads), the
+ * Poisson / spectral Helmholtz band solve (column pairs per block: 64, 128)
+ * and the projection (block of j by i: 32x2, 32x4, 32x8, 64x2).  cf_create
+ * times the candidates on the new instance (before it holds state) and keeps the fastest; cf_batch_create does the same on
  * the batch's own launches with their outputs in scratch memory.  Results
  * are cached per configuration (per member set for a batch) for the process
  * and, when the environment variable CF_TUNE_CACHE names a file, across

@@ -317,7 +317,7 @@ class Instance:
         return r == 1
 
     def launch_shape(self):
-        """Tuned launch shape: (back-substitution threads, Poisson threads,
+        """Tuned launch shape: (line-solve threads, Poisson threads,
         projection block x, projection block y)."""
         out = (ctypes.c_int * 4)()
         _check(self.L.cf_get_launch_shape(self.h, out), "cf_get_launch_shape")
