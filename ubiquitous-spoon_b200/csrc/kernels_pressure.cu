@@ -383,11 +383,12 @@ __device__ __forceinline__ void k_div_fftx_body(const Geo& G, const DivArgs& A, 
     }
 }
 
-// Blocks per SM: 4 up to 192 (64 registers; with 5 the loads in flight
-// do not fit, 47 -> 52 us at 192 x 192 x 128), 3 at 320 and 384 (60 -> 55 us at
-// 320 x 384 x 48), 2 where the size is planned (3: 69 -> 82 us at 300 x 384 x 48).
+// Blocks per SM: 4 up to 192 (64 registers; with 5 the loads in flight do not
+// fit, 47 -> 52 us at 192 x 192 x 128, order 2), above it 3 at order 2 (2: 55 ->
+// 60 us at 320 x 384 x 48) and 2 at order 4 (3: 83 -> 107), 2 where the size is
+// planned (3: 69 -> 82 us at 300 x 384 x 48).
 template <int ORDER, int N>
-__global__ void __launch_bounds__(FFT_THREADS, N == 0 ? 2 : N <= 192 ? 4 : 3) k_div_fftx(Geo G, DivArgs A)
+__global__ void __launch_bounds__(FFT_THREADS, N == 0 || (N > 192 && ORDER == 4) ? 2 : N <= 192 ? 4 : 3) k_div_fftx(Geo G, DivArgs A)
 {
     k_div_fftx_body<ORDER, N>(G, A, blockIdx);
 }
