@@ -95,6 +95,26 @@ def test_batch_step_equals_alone(cf, gpu):
         inst.close()
 
 
+# columns walked whole (more than 192 rows, or a plane of more tiles than
+# three quarters of the SMs): power-of-two, fixed and planned transforms, odd planes
+WHOLE = [(2, 64, 48, 200, 2800.0), (4, 64, 48, 200, 2800.0), (4, 30, 45, 193, 4000.0), (2, 9, 25, 193, 4000.0),
+         (4, 200, 160, 9, 5000.0), (2, 192, 192, 20, 5000.0), (4, 128, 256, 40, 8000.0)]
+
+
+@pytest.mark.parametrize("member", WHOLE)
+def test_batch_member_is_the_plain_path_bit_for_bit(cf, gpu, member):
+    """A member's fields, pressure and log equal those of the same instance
+    stepped on its own, whatever instantiation of a kernel each goes through."""
+    a, b = make(cf, *member, seed=3), make(cf, *member, seed=3)
+    a.step(7)
+    a.sync()
+    cf.batch_step([b], 7)
+    b.sync()
+    assert_same(a, b)
+    a.close()
+    b.close()
+
+
 def test_batch_rejects_foreign_steps_and_schemes(cf, gpu):
     a = make(cf, 2, 64, 64, 16, 2800.0, 1)
     b = make(cf, 2, 64, 64, 16, 2800.0, 2)

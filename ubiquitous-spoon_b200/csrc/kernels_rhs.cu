@@ -14,6 +14,7 @@
 #include "host_band.h"
 #include "wall.cuh"
 #include "batch.cuh"
+#include "rounding.cuh"
 
 #include <algorithm>
 #include <type_traits>
@@ -63,10 +64,10 @@ __device__ __forceinline__ void ghosts_body(const Geo& G, const GhostArgs& A, ui
     at(wt) = t1;
     if (ORDER == 4) {
         // EXTRAP: massflux4 wall extrapolation (advect.c:108-109, 124-125)
-        at(kb - 1) = EXTRAP ? 2.0 * b1 - x0 : b2;
-        at(kb - 2) = EXTRAP ? 2.0 * b1 - x1 : b3;
-        at(wt + 1) = EXTRAP ? 2.0 * t1 - y0 : t2;
-        at(wt + 2) = EXTRAP ? 2.0 * t1 - y1 : t3;
+        at(kb - 1) = EXTRAP ? mad(2.0, b1, -x0) : b2;
+        at(kb - 2) = EXTRAP ? mad(2.0, b1, -x1) : b3;
+        at(wt + 1) = EXTRAP ? mad(2.0, t1, -y0) : t2;
+        at(wt + 2) = EXTRAP ? mad(2.0, t1, -y1) : t3;
     }
 }
 
@@ -206,10 +207,6 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // pairs of points
 __device__ __forceinline__ double2 ld2(const double* p) { return *reinterpret_cast<const double2*>(p); }
 __device__ __forceinline__ void st2(double* p, double2 v) { *reinterpret_cast<double2*>(p) = v; }
-__device__ __forceinline__ double2 operator+(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 operator-(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ double2 operator*(double2 a, double2 b) { return make_double2(a.x * b.x, a.y * b.y); }
-__device__ __forceinline__ double2 operator*(double a, double2 b) { return make_double2(a * b.x, a * b.y); }
 
 // Halved interpolation to the face between a0 and a1 (massflux{x,y,z}{2,4},
 // advect.c:6-283, with the 0.5 of the advected face value).
@@ -381,7 +378,7 @@ __device__ __forceinline__ void rhs_field(const Geo& G, const RhsArgs& A, const 
         zw[LO + NZ] = ld2(ringat(F, k + NZ));
         auto Z = [&](int d) { return LO + d >= 0 ? zw[LO + d >= 0 ? LO + d : 0] : ld2(ringat(F, k + d)); };
         const double2 q0 = Z(0);
-        const double2 gk = make_double2(gnext.x + shift, gnext.y + shift);
+        const double2 gk = gnext + make_double2(shift, shift);
         if (k + 1 < T.ke) gnext = load_g(k + 1, gio + T.plane);
 
         // ---- plane k: x neighbours, y neighbours (columns j-4 .. j+5)
@@ -400,13 +397,20 @@ __device__ __forceinline__ void rhs_field(const Geo& G, const RhsArgs& A, const 
         // add_laplacexy_operator_{u,w}{2,4} (diffuseu.c:286-359, diffusew.c:290-363)
         double2 lap;
         if (ORDER == 2) {
-            lap = diff * (idx2 * (X(1) - 2.0 * q0 + X(-1)) + idy2 * (Y(1) - 2.0 * q0 + Y(-1)));
+            lap = idx2 * (X(1) - 2.0 * q0 + X(-1)) + idy2 * (Y(1) - 2.0 * q0 + Y(-1));
         } else {
             const double lapc = -2.0 * (L1 + L2 + L3) * (idx2 + idy2);
             const double2 lx = L3 * (X(3) + X(-3)) + L2 * (X(2) + X(-2)) + L1 * (X(1) + X(-1));
             const double2 ly = L3 * (Y(3) + Y(-3)) + L2 * (Y(2) + Y(-2)) + L1 * (Y(1) + Y(-1));
-            lap = diff * ((idx2 * lx + idy2 * ly) + lapc * q0);
+            lap = (idx2 * lx + idy2 * ly) + lapc * q0;
         }
+        // the explicit diffusion enters first at order 2 and last at order 4, by measurement (64 x 64 x 384
+        // 413 -> 399 us, 256 x 256 x 192 at order 4 the other way round 619 -> 626)
+        if (MODE == RHS_CHANNEL) lap = diff * lap;
+        auto onto_lap = [&](Product2 advection) -> double2 {
+            if (MODE == RHS_CHANNEL || ORDER == 4) return advection;
+            return advection + diff * lap;
+        };
 
         // ---- faces for the other fields, and the flux of the field's own direction
         const int wat = T.ty * RT_J + T.jl, uat = (T.ty + 2) * RT_J + T.jl, vat = T.ty * (RT_J + 4) + T.jl + 2;
@@ -425,7 +429,7 @@ __device__ __forceinline__ void rhs_field(const Geo& G, const RhsArgs& A, const 
             // faces j-2 .. j+2, each once for both points
             const double2 e0 = face<ORDER>(Y(-3), Y(-2), Y(-1), q0);                     // faces -2, -1
             const double2 e2 = face<ORDER>(Y(-1), q0, Y(1), Y(2));                       // faces 0, 1
-            const double e4 = ORDER == 4 ? B1h * (Y(2).x + Y(3).x) + B2h * (Y(1).x + Y(3).y) : 0.0;   // face 2
+            const double e4 = ORDER == 4 ? dot(B2h, add(Y(1).x, Y(3).y), B1h, add(Y(2).x, Y(3).x)) : 0.0;   // face 2
             own = flux<ORDER>(e0, make_double2(e0.y, e2.x), e2, make_double2(e2.y, e4), Y(-3), Y(-1), q0, Y(1), Y(3));
         } else if (F == 2) {
             if (ORDER == 2) {   // plane k: the z fluxes use m(k)
@@ -468,21 +472,27 @@ __device__ __forceinline__ void rhs_field(const Geo& G, const RhsArgs& A, const 
         }
 
         double2 f;
-        if (F == 3) {   // flux_quick + advect_scalar (scalar.c:79-162): no faces of others
+        // flux_quick + advect_scalar (scalar.c:79-162): no faces of others.  At order 2
+        // the longest work of a row, done while the other fields form their fluxes
+        // (64 x 64 x 384 449 -> 413 us); at order 4 before the barrier, beside the
+        // velocities' own longer halves (after it 256 x 256 x 192 619 -> 687 us).
+        auto scalar = [&]() {
             const double* u = ringat(0, k);
             const double* v = ringat(1, k);
             const double2 va = ld2(v - 2), vb = ld2(v);
             const double2 kx0 = curv(X(1), q0, X(-1)), ky0 = curv(Y(1), q0, Y(-1)), kzp = curv(Z(2), Z(1), q0);
-            const double2 fxp = quick(DYDZ(0) * ld2(u), q0, X(1), kx0, curv(X(2), X(1), q0));
-            const double2 fxm = quick(DYDZ(0) * ld2(u - PJ), X(-1), q0, curv(q0, X(-1), X(-2)), kx0);
-            const double2 fyp = quick(DXDZ(0) * vb, q0, Y(1), ky0, curv(Y(2), Y(1), q0));
-            const double2 fym = quick(DXDZ(0) * make_double2(va.y, vb.x), Y(-1), q0, curv(q0, Y(-1), Y(-2)), ky0);
+            const Product2 fxp = quick(DYDZ(0) * ld2(u), q0, X(1), kx0, curv(X(2), X(1), q0));
+            const Product2 fxm = quick(DYDZ(0) * ld2(u - PJ), X(-1), q0, curv(q0, X(-1), X(-2)), kx0);
+            const Product2 fyp = quick(DXDZ(0) * vb, q0, Y(1), ky0, curv(Y(2), Y(1), q0));
+            const Product2 fym = quick(DXDZ(0) * make_double2(va.y, vb.x), Y(-1), q0, curv(q0, Y(-1), Y(-2)), ky0);
             const double2 fzp = quick(dxdy * ld2(ringat(2, k)), q0, Z(1), kz, kzp);
-            f = (-mrow[8]) * ((fxp - fxm) + (fyp - fym) + (fzp - fz));
+            f = onto_lap((-mrow[8]) * ((fxp - fxm) + (fyp - fym) + (fzp - fz)));
             kz = kzp;
             fz = fzp;
-        }
+        };
+        if (F == 3 && ORDER == 4) scalar();
         __syncthreads();   // the row's faces are in place
+        if (F == 3 && ORDER == 2) scalar();
 
         if (F < 3) {
             double2 other;   // the flux (for w: both) of the directions whose faces others hold
@@ -528,10 +538,10 @@ __device__ __forceinline__ void rhs_field(const Geo& G, const RhsArgs& A, const 
                 }
                 mz = mup;
             }
-            const double2 zs = ORDER == 2 ? dxdy * (zph - zmh) : dxdy * (A1 * (zph - zmh) + A2 * (zp3 - zm3));
-            if (F == 0) f = (-mrow[8]) * ((DYDZ(0) * own + DXDZ(0) * other) + zs);
-            if (F == 1) f = (-mrow[8]) * ((DYDZ(0) * other + DXDZ(0) * own) + zs);
-            if (F == 2) f = (-mrow[9]) * (other + zs);
+            const double2 zs = ORDER == 2 ? zph - zmh : A1 * (zph - zmh) + A2 * (zp3 - zm3);
+            if (F == 0) f = onto_lap((-mrow[8]) * ((DYDZ(0) * own + DXDZ(0) * other) + dxdy * zs));
+            if (F == 1) f = onto_lap((-mrow[8]) * ((DYDZ(0) * other + DXDZ(0) * own) + dxdy * zs));
+            if (F == 2) f = onto_lap((-mrow[9]) * (other + dxdy * zs));
             // add_buoyancy{2,4} (scalar.c:6-76); skipped when every betg is zero
             if (buoyancy) {
                 const double* c = ringat(3, k);
@@ -552,7 +562,7 @@ __device__ __forceinline__ void rhs_field(const Geo& G, const RhsArgs& A, const 
                 }
             }
         }
-        if (MODE != RHS_CHANNEL) f = f + lap;
+        if (MODE != RHS_CHANNEL && ORDER == 4) f = f + diff * lap;
 
         // ---- right-hand side of the implicit solve, rows GZ .. (u, v, c: nz rows; w: nz - 1 faces)
         const double2* r2 = reinterpret_cast<const double2*>(cst + (k & 1) * RT_FWMAX);
@@ -566,8 +576,7 @@ __device__ __forceinline__ void rhs_field(const Geo& G, const RhsArgs& A, const 
             }
         }
         double2 h = r[2 * HH + 1] * f + r[2 * HH + 2] * gk;
-        h.x += r[2 * HH + 3];
-        h.y += r[2 * HH + 3];
+        h = h + make_double2(r[2 * HH + 3], r[2 * HH + 3]);
         // the old w beyond its wall faces is apply_bc_w's (the ring holds the massflux4 extrapolation)
         double2 b1 = z2, b2 = z2;
         if (WALL && F == 2 && ORDER == 4) {

@@ -17,6 +17,7 @@
 #include "host_band.h"
 #include "wall.cuh"
 #include "batch.cuh"
+#include "rounding.cuh"
 
 namespace cf {
 
@@ -131,14 +132,11 @@ __device__ __forceinline__ void line_chunks(const Geo& G, const SolveArgs& A, ui
     // one row: the newest value enters last
     auto step = [](double2 v, double k1, double k2, double k3, double2& a1, double2& a2, double2& a3) {
         if (ORDER == 4) {
-            v.x = (v.x - k3 * a3.x) - k2 * a2.x;
-            v.y = (v.y - k3 * a3.y) - k2 * a2.y;
+            v = (v - k3 * a3) - k2 * a2;
             a3 = a2;
             a2 = a1;
         }
-        v.x -= k1 * a1.x;
-        v.y -= k1 * a1.y;
-        return a1 = v;
+        return a1 = v - k1 * a1;
     };
     // coefficients of rows r and r + 1 (r even)
     auto rows2 = [&](const double2* T, int r, double (&k)[6]) {
@@ -174,18 +172,15 @@ __device__ __forceinline__ void line_chunks(const Geo& G, const SolveArgs& A, ui
             const double2 e1 = ends[(q * H + 0) * lanes + lc];
             double2* to = hist + (q + dir) * H * lanes + lc;
             if (ORDER == 2) {
-                b1 = make_double2(e1.x + M[q] * b1.x, e1.y + M[q] * b1.y);
+                b1 = e1 + M[q] * b1;
             } else {
                 const double2 e2 = ends[(q * H + 1) * lanes + lc], e3 = ends[(q * H + 2) * lanes + lc];
                 const double2* m = reinterpret_cast<const double2*>(M + q * MS);
                 const double2 m01 = m[0], m23 = m[1], m45 = m[2], m67 = m[3];
                 const double m8 = m[4].x;
-                const double2 c1 = make_double2((e1.x + m01.x * b1.x) + (m01.y * b2.x + m23.x * b3.x),
-                                                (e1.y + m01.x * b1.y) + (m01.y * b2.y + m23.x * b3.y));
-                const double2 c2 = make_double2((e2.x + m23.y * b1.x) + (m45.x * b2.x + m45.y * b3.x),
-                                                (e2.y + m23.y * b1.y) + (m45.x * b2.y + m45.y * b3.y));
-                b3 = make_double2((e3.x + m67.x * b1.x) + (m67.y * b2.x + m8 * b3.x),
-                                  (e3.y + m67.x * b1.y) + (m67.y * b2.y + m8 * b3.y));
+                const double2 c1 = (e1 + m01.x * b1) + (m01.y * b2 + m23.x * b3);
+                const double2 c2 = (e2 + m23.y * b1) + (m45.x * b2 + m45.y * b3);
+                b3 = (e3 + m67.x * b1) + (m67.y * b2 + m8 * b3);
                 b1 = c1;
                 b2 = c2;
                 to[1 * lanes] = b2;
@@ -310,9 +305,7 @@ __device__ __forceinline__ void line_chunks(const Geo& G, const SolveArgs& A, ui
 #pragma unroll
     for (int r = 0; r < R; r++)
         if (r < size) {
-            const double d = __ldg(dz + r);
-            bulk.x += h[r].x * d;
-            bulk.y += h[r].y * d;
+            bulk = bulk + __ldg(dz + r) * h[r];
         }
     const double sum = oct_sum((v0 ? bulk.x : 0.0) + (v1 ? bulk.y : 0.0));
     double* sums = reinterpret_cast<double*>(hist);   // last read before the last barrier
@@ -351,11 +344,11 @@ __device__ __forceinline__ void back_column(const Geo& G, const SolveArgs& A, ui
             if (i >= 0) {
                 double y = p[u];
                 if (i - PD >= 0) p[u] = s[(i - PD) * P];
-                if (ORDER == 4) y = (y - __ldg(rows + i * H + 2) * y3) - __ldg(rows + i * H + 1) * y2;
-                y -= __ldg(rows + i * H) * y1;   // y1 last
+                if (ORDER == 4) y = msub(__ldg(rows + i * H + 1), y2, msub(__ldg(rows + i * H + 2), y3, y));
+                y = msub(__ldg(rows + i * H), y1, y);   // y1 last
                 y3 = y2; y2 = y1; y1 = y;
                 if (valid) x[(GZ + i) * P] = y;
-                if (STATS) bulk += y * __ldg(dz + i);
+                if (STATS) bulk = mad(y, __ldg(dz + i), bulk);
             }
         }
     }
@@ -395,8 +388,8 @@ __device__ __forceinline__ void control_finish(const MassArgs& A, long long cnt,
     double s[4];
     s[0] = mean;
     if (A.order == 4) {
-        s[1] = A.kappa * (A1 * (bot[2] - bot[1]) + A2 * (bot[3] - bot[0])) / (0.5 * (dz[g] + dz[g - 1]));
-        s[2] = A.kappa * (A1 * (top[2] - top[1]) + A2 * (top[3] - top[0])) / (0.5 * (dz[n2 - g] + dz[n2 - g - 1]));
+        s[1] = mul(A.kappa, dot(A1, bot[2] - bot[1], A2, bot[3] - bot[0])) / (0.5 * (dz[g] + dz[g - 1]));
+        s[2] = mul(A.kappa, dot(A1, top[2] - top[1], A2, top[3] - top[0])) / (0.5 * (dz[n2 - g] + dz[n2 - g - 1]));
     } else {
         s[1] = A.kappa * (bot[2] - bot[1]) / (0.5 * (dz[g] + dz[g - 1]));
         s[2] = A.kappa * (top[2] - top[1]) / (0.5 * (dz[n2 - g] + dz[n2 - g - 1]));
@@ -407,7 +400,7 @@ __device__ __forceinline__ void control_finish(const MassArgs& A, long long cnt,
     // anywhere in it (or in the control) shows here; the flag stays set
     // until the host resets it with new fields.
     if (A.nonfinite && !isfinite(s[0] + m)) *A.nonfinite = 1.0;
-    for (int t = 0; t < 4; t++) s[t] += A.green[t] * m;
+    for (int t = 0; t < 4; t++) s[t] = mad(A.green[t], m, s[t]);
     *A.m_out = m;
     if (A.log_base) {
         double* row = A.log_base + (cnt % A.log_cap) * LOG_COLS + A.col;
@@ -488,7 +481,7 @@ __device__ __forceinline__ void control_body(const ControlArgs& A, uint3 bid)
         double s[LINE_STATS];
 #pragma unroll
         for (int e = 0; e < LINE_STATS; e++) s[e] = __ldcg(A.sums + q * LINE_STATS + e);
-        control_finish(A.m[q], cnt, s[0] * A.ilz, s + 1, s + 5, 0.5 * (s[9] + s[10]));
+        control_finish(A.m[q], cnt, mul(s[0], A.ilz), s + 1, s + 5, 0.5 * (s[9] + s[10]));
     }
     if (threadIdx.x == 0) {
         *A.m[1].counter = cnt + 1;
