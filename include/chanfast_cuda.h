@@ -216,9 +216,7 @@ int cf_z_coords(const cf_instance *inst, double *zp, double *zw);         /* get
  * in device memory: geometry, arguments, own grid).  Members may differ in
  * grid size, order and physical parameters; they must use
  * CF_SCHEME_CHANFAST and live on one device.  Each member's results are the
- * same, bit for bit, whatever the other members are, and agree with stepping
- * it alone with cf_step to rounding (a batch solves whole columns, where
- * cf_step cuts the columns of a small plane into chunks).
+ * same, bit for bit, as stepping it alone with cf_step.
  *
  * cf_batch_step: advance every member by nsub substeps on `stream` (NULL:
  * the first member's stream), recording the launches on the spot.  Ordered

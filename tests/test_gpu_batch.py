@@ -6,9 +6,9 @@ Alone and in the mix: each member's fields, pressure and log equal, bit for
 bit, the same instance stepped alone in a batch of one (the same kernels on
 the same arguments; neighbours in a launch do not interact).  Against the
 plain single-instance path (cf_step), whose kernels are separate
-instantiations of the same bodies and may contract a few multiply-adds
-differently, they agree to relative L2 <= 1e-13 (the engine's own bar against
-the reference is 1e-13 on u, v, w, c)."""
+instantiations of the same bodies: bit for bit too (rounding.cuh), and in the
+longer mixed runs to relative L2 <= 1e-13 (the engine's own bar against the
+reference is 1e-13 on u, v, w, c)."""
 import numpy as np
 import pytest
 
@@ -101,7 +101,13 @@ WHOLE = [(2, 64, 48, 200, 2800.0), (4, 64, 48, 200, 2800.0), (4, 30, 45, 193, 40
          (4, 200, 160, 9, 5000.0), (2, 192, 192, 20, 5000.0), (4, 128, 256, 40, 8000.0)]
 
 
-@pytest.mark.parametrize("member", WHOLE)
+# partitioned columns (chunks of 16 rows): one short chunk, a last chunk of one
+# row, the tallest; row blocks of every length in k_rhs; odd planes
+PARTITIONED = [(2, 64, 64, 64, 2800.0), (4, 64, 64, 64, 2800.0), (2, 24, 30, 8, 3000.0), (4, 48, 40, 17, 3000.0),
+               (4, 90, 75, 53, 5000.0), (2, 9, 25, 33, 5000.0), (2, 128, 128, 43, 5000.0), (4, 64, 48, 192, 5000.0)]
+
+
+@pytest.mark.parametrize("member", WHOLE + PARTITIONED)
 def test_batch_member_is_the_plain_path_bit_for_bit(cf, gpu, member):
     """A member's fields, pressure and log equal those of the same instance
     stepped on its own, whatever instantiation of a kernel each goes through."""
@@ -113,6 +119,22 @@ def test_batch_member_is_the_plain_path_bit_for_bit(cf, gpu, member):
     assert_same(a, b)
     a.close()
     b.close()
+
+
+def test_members_in_the_mix_are_the_plain_path_bit_for_bit(cf, gpu):
+    """The same with other members about: they change the rows that a block of
+    a member's right-hand side takes (its share of the GPU), not its results."""
+    members = MEMBERS + PARTITIONED + WHOLE[:2]
+    alone, mixed = ([make(cf, *m, seed=q) for q, m in enumerate(members)] for _ in range(2))
+    with cf.Batch(mixed) as B:
+        B.run(3)
+        B.sync()
+    for a, b in zip(alone, mixed):
+        a.step_graph(3)
+        a.sync()
+        assert_same(a, b)
+    for inst in alone + mixed:
+        inst.close()
 
 
 def test_batch_rejects_foreign_steps_and_schemes(cf, gpu):

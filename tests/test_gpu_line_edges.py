@@ -57,8 +57,8 @@ def test_substeps_match_restatement(cf, gpu, order, nx, ny, nz):
 
 
 def test_batch_of_odd_and_even_planes_matches_plain(cf, gpu):
-    """A batch runs whole columns whatever the plain path does, odd and even
-    planes in launches of their own: against the plain path to rounding."""
+    """Odd and even planes, partitioned and whole columns, in launches of their
+    own: against the plain path (test_gpu_batch.py: bit for bit)."""
     out = []
     for batched in (False, True):
         insts = []

@@ -278,6 +278,7 @@ constexpr int RHS_MIN_ROWS = 6;      // fewest rows of a k_rhs block (its wall c
 long long rhs_tiles(const Geo& G);
 int rhs_chunk(const Geo& G, int sms, bool sweep);
 int line_threads(const Geo& G);
+int line_batch_threads(const Geo& G);
 dim3 grid_line(const Geo& G);
 size_t line_smem(const Geo& G);
 dim3 grid_div(const Geo& G);                       // power-of-two nx: divergence
@@ -289,8 +290,13 @@ dim3 grid_c2r(const Geo& G, int nrows, int nfields);
 dim3 grid_project(const Geo& G);
 bool batch_pow2(int n);                            // n has a power-of-two transform kernel
 void launch_ghosts_batch(const BatchLaunch& L, int order, cudaStream_t st);
-void launch_rhs_batch(const BatchLaunch& L, int key, cudaStream_t st);   // key: order, + 8 for odd ny
-void launch_line_batch(const BatchLaunch& L, int order, cudaStream_t st);
+// keys: order, + 8 for odd ny (k_rhs), + 16 for partitioned line solves (k_line; k_rhs at order 4)
+inline int rhs_batch_key(const Geo& G)
+{
+    return G.order + (G.ny % 2 ? 8 : 0) + (G.order == 4 && G.partitioned ? 16 : 0);
+}
+void launch_rhs_batch(const BatchLaunch& L, int key, cudaStream_t st);
+void launch_line_batch(const BatchLaunch& L, int key, cudaStream_t st);
 void launch_control_batch(const BatchLaunch& L, cudaStream_t st);
 void launch_div_batch(const BatchLaunch& L, int order, cudaStream_t st);
 void launch_r2c_batch(const BatchLaunch& L, int nx, cudaStream_t st);

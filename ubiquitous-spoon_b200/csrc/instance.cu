@@ -432,6 +432,7 @@ struct cf_instance {
     double* avg = nullptr;          // channel scheme: xy-averages of u
     double* avg_c = nullptr;        // and of c
     int rhs_rows = 0;               // rows per k_rhs block (rhs_chunk)
+    int sms = 0;                    // of the device
     double* dscal = nullptr;        // [0] mdpdx, [1] dcdt, [2] non-finite flag, [3] copy-wait fault flag
     // channel scheme with the fused Helmholtz solves: device records [3][4]
     // (substep set, field u v w c) of k_poisson_fft_batch without FILL
@@ -463,9 +464,11 @@ struct cf_instance {
 
 namespace {
 
-// Whether an instance on its own runs its line solves partitioned (k_line does
+// Whether an instance runs its line solves partitioned (k_line does
 // both sweeps, k_rhs takes any number of rows a block) or with the forward
-// sweep in k_rhs, up whole columns, and k_line walking back down.  The
+// sweep in k_rhs, up whole columns, and k_line walking back down.  The two
+// differ in rounding; an instance takes the same one on its own and in a batch,
+// so that its results do not depend on how it is stepped.  The
 // partition is for planes too small to give every SM a k_rhs tile: k_rhs then
 // gets its blocks from the rows, and k_line's threads walk 16 rows instead of
 // all.  Measured, k_rhs + k_line in us, partitioned against whole columns:
@@ -476,7 +479,7 @@ namespace {
 // other streams, which fills those, is slowed (256 x 256 x 192 at order 4,
 // three instances at once: 8.54 against 8.32 ms).  Above 192 rows the carries
 // through the chunks cost more than the walk (512 x 512 x 384: 2880 against
-// 1480 us).  In a batch the other members fill the GPU: whole columns.
+// 1480 us).
 bool line_partitioned(bool channel, const Geo& G, int sms)
 {
     return !channel && G.nz <= LINE_MAX_ROWS && 4 * rhs_tiles(G) <= 3 * sms;
@@ -1029,15 +1032,9 @@ int build_helm_records(cf_instance* I)
     return CF_OK;
 }
 
-// A member's geometry in a batch: its line solves are not partitioned there
-// (line_partitioned).
-Geo whole_columns(Geo G)
-{
-    G.partitioned = false;
-    return G;
-}
-
 struct BatchSink : Sink {
+    std::map<int, long long> tiles;   // k_rhs tiles of all members in a launch, by rhs_batch_key
+    int sms = 1;
     std::vector<BatchStage> stages;
     size_t cursor = 0;
     bool mismatch = false;
@@ -1060,23 +1057,19 @@ struct BatchSink : Sink {
     }
     void rhs(const Geo& G, const RhsArgs& A) override
     {
-        const Geo W = whole_columns(G);
+        // row blocks for the member's share of the SMs in its launch, by tiles
         RhsArgs B = A;
-        B.chunk = G.nz;
-        next(ST_RHS).rhs.push_back(batch_rec(W, B, grid_rhs(W, B.chunk)));
+        const long long share = std::max(1ll, sms * rhs_tiles(G) / tiles[rhs_batch_key(G)]);
+        B.chunk = rhs_chunk(G, (int) share, !G.partitioned);
+        next(ST_RHS).rhs.push_back(batch_rec(G, B, grid_rhs(G, B.chunk)));
     }
     void line(const Geo& G, const SolveBatch& A) override
     {
-        const Geo W = whole_columns(G);
-        SolveBatch B = A;
-        for (SolveArgs& S : B.a) S.ngroups = line_groups(W);
-        next(ST_LINE).line.push_back(batch_rec(W, B, grid_line(W)));
+        next(ST_LINE).line.push_back(batch_rec(G, A, grid_line(G)));
     }
     void control(const Geo& G, const ControlArgs& A) override
     {
-        ControlArgs B = A;
-        B.ngroups = line_groups(whole_columns(G));
-        next(ST_CONTROL).control.push_back(batch_rec(G, B, dim3(2 * LINE_STATS)));
+        next(ST_CONTROL).control.push_back(batch_rec(G, A, dim3(2 * LINE_STATS)));
     }
     void div_fftx(const Geo& G, const DivArgs& A) override
     {
@@ -1171,12 +1164,22 @@ void add_groups(BatchProgram& P, int kernel, const std::vector<BatchRec<Args>>& 
     }
 }
 
+// The line solves of a batch: members with partitioned solves and those
+// without in launches of their own.
+void add_line_groups(BatchProgram& P, const std::vector<BatchRec<SolveBatch>>& recs)
+{
+    for (const bool part : {false, true}) {
+        std::vector<BatchRec<SolveBatch>> some;
+        for (const auto& r : recs)
+            if (r.G.partitioned == part) some.push_back(r);
+        if (some.empty()) continue;
+        add_groups(P, BK_LINE, some, [](const auto& r) { return r.G.order + (r.G.partitioned ? 16 : 0); },
+                   [](const auto& r) { return line_smem(r.G); }, dim3(line_batch_threads(some[0].G)));
+    }
+}
+
 // Block shape of a batched launch of a tuned kernel: every record of a batch
 // is recorded with the batch's one launch shape (record()).
-dim3 line_block(const std::vector<BatchRec<SolveBatch>>& r)
-{
-    return dim3(r.empty() ? 128 : line_threads(r[0].G));
-}
 dim3 poisson_block(const std::vector<BatchRec<PoissonArgs>>& r)
 {
     return dim3(r.empty() ? 128 : r[0].G.shape.pois_threads);
@@ -1198,8 +1201,8 @@ void compile(const BatchSink& K, BatchProgram& P)
     for (const BatchStage& S : K.stages) {
         switch (S.kind) {
         case ST_GHOSTS: add_groups(P, BK_GHOSTS, S.ghosts, order, none); break;
-        case ST_RHS: add_groups(P, BK_RHS, S.rhs, [](const auto& r) { return r.G.order + (r.G.ny % 2 ? 8 : 0); }, none); break;
-        case ST_LINE: add_groups(P, BK_LINE, S.line, order, none, line_block(S.line)); break;
+        case ST_RHS: add_groups(P, BK_RHS, S.rhs, [](const auto& r) { return rhs_batch_key(r.G); }, none); break;
+        case ST_LINE: add_line_groups(P, S.line); break;
         case ST_CONTROL: add_groups(P, BK_CONTROL, S.control, none, none); break;
         case ST_DIV:
             add_groups(P, BK_DIV, S.div, order, none);
@@ -1256,9 +1259,12 @@ void run_program(const BatchProgram& P, cudaStream_t st)
 int record_sink(const std::vector<cf_instance*>& v, int nsub, const LaunchShape& shape, BatchSink& K)
 {
     std::vector<LaunchShape> own;
+    K.tiles.clear();
+    K.sms = std::max(1, v[0]->sms);
     for (cf_instance* I : v) {
         own.push_back(I->geo.shape);
         I->geo.shape = shape;
+        K.tiles[rhs_batch_key(I->geo)] += rhs_tiles(I->geo);
     }
     int rc = CF_OK;
     for (int q = 0; q < nsub && rc == CF_OK; q++) {
@@ -1682,7 +1688,7 @@ int tune_batch(const std::vector<cf_instance*>& v, cudaStream_t st, LaunchShape&
         if (kind == 0) {
             auto recs = line;
             for (auto& r : recs) { r.G.shape = sh; dim3 g = grid_line(r.G); r.gx = g.x; r.gy = g.y; r.gz = g.z; }
-            add_groups(P, BK_LINE, recs, order, none, line_block(recs));
+            add_line_groups(P, recs);
         } else if (kind == 1) {
             auto recs = pois;
             for (auto& r : recs) { r.G.shape = sh; dim3 g = grid_poisson(r.G); r.gx = g.x; r.gy = g.y; r.gz = g.z; }
@@ -1765,9 +1771,8 @@ static int create_impl(const cf_config* cfg, void* stream, cf_instance* I)
     G.nkx = C.nx / 2 + 1;
     G.plane = (long long) C.nx * C.ny;
     G.splane = (long long) G.nkx * C.ny;
-    int sms = 0;
-    CF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, I->device));
-    G.partitioned = line_partitioned(C.scheme == CF_SCHEME_CHANNEL, G, sms);
+    CF_CUDA(cudaDeviceGetAttribute(&I->sms, cudaDevAttrMultiProcessorCount, I->device));
+    G.partitioned = line_partitioned(C.scheme == CF_SCHEME_CHANNEL, G, I->sms);
     G.dx = I->m.dx;
     G.dy = I->m.dy;
     G.dxdy = I->m.dx * I->m.dy;
@@ -1806,7 +1811,7 @@ static int create_impl(const cf_config* cfg, void* stream, cf_instance* I)
     CF_CUDA(cudaMalloc(&I->partial_c, nsum * sizeof(double)));
     CF_CUDA(cudaMalloc(&I->csum, (2 * LINE_STATS + 1) * sizeof(double)));
     CF_CUDA(cudaMemsetAsync(I->csum, 0, (2 * LINE_STATS + 1) * sizeof(double), I->stream));
-    I->rhs_rows = rhs_chunk(G, std::max(sms, 1), C.scheme != CF_SCHEME_CHANNEL && !G.partitioned);
+    I->rhs_rows = rhs_chunk(G, std::max(I->sms, 1), C.scheme != CF_SCHEME_CHANNEL && !G.partitioned);
     CF_CUDA(cudaMalloc(&I->avg, (size_t) G.n2 * sizeof(double)));
     CF_CUDA(cudaMalloc(&I->avg_c, (size_t) G.n2 * sizeof(double)));
     CF_CUDA(cudaMalloc(&I->dscal, 8 * sizeof(double)));

@@ -169,7 +169,10 @@ constexpr double B1h = 0.5 * B1, B2h = 0.5 * B2;   // halved interpolation weigh
 constexpr double L1 = A1 * A1 - 2.0 * A1 * A2, L2 = 2.0 * A1 * A2, L3 = A2 * A2;
 
 constexpr int RT_FWMAX = 14;  // widest fused row (order 4: 13), padded to 16-byte pairs
-constexpr int RT_MROW = 12;   // per-row grid metrics: dydz[k-1..k+2], dxdz[k-1..k+2], ivol[k], ivolw[k] (+2 pad)
+// per-row grid metrics: dydz[k-1..k+2], dxdz[k-1..k+2], ivol[k], ivolw[k], and with RCS a field's scalars
+template <bool RCS>
+constexpr int RT_MROW = RCS ? 16 : 12;
+constexpr int RM_DXDY = 10, RM_DIFF = 11, RM_SHIFT = 12, RM_IDX2 = 13, RM_IDY2 = 14;
 // face buffers: u's with rows i0-2 .. i0+8, v's with columns j0-2 .. j0+33, w's on the tile
 constexpr int RF_U = (RT_I + 3) * RT_J, RF_V = RT_I * (RT_J + 4), RF_W = RT_I * RT_J;
 constexpr int RF_UY = 0, RF_UZ = RF_U, RF_VX = 2 * RF_U, RF_VZ = 2 * RF_U + RF_V, RF_WX = 2 * RF_U + 2 * RF_V,
@@ -180,14 +183,14 @@ template <int ORDER>
 __host__ __device__ constexpr int rhs_faces() { return 4 * RhsTile<ORDER>::FIELD; }
 template <int ORDER>
 __host__ __device__ constexpr int rhs_rows() { return rhs_faces<ORDER>() + 2 * RF_ALL; }
-template <int ORDER>
-__host__ __device__ constexpr int rhs_queue() { return rhs_rows<ORDER>() + 4 * 2 * (RT_FWMAX + RT_MROW); }
-template <int ORDER>
-__host__ __device__ constexpr int rhs_offs() { return rhs_queue<ORDER>() + (ORDER == 4 ? 4 * 2 * RT_THREADS : 0); }
-template <int ORDER>
+template <int ORDER, bool RCS>
+__host__ __device__ constexpr int rhs_queue() { return rhs_rows<ORDER>() + 4 * 2 * (RT_FWMAX + RT_MROW<RCS>); }
+template <int ORDER, bool RCS>
+__host__ __device__ constexpr int rhs_offs() { return rhs_queue<ORDER, RCS>() + (ORDER == 4 ? 4 * 2 * RT_THREADS : 0); }
+template <int ORDER, bool RCS = false>
 constexpr size_t rhs_smem_bytes()
 {
-    return (size_t) rhs_offs<ORDER>() * sizeof(double) + RhsTile<ORDER>::PLANE * sizeof(int);
+    return (size_t) rhs_offs<ORDER, RCS>() * sizeof(double) + RhsTile<ORDER>::PLANE * sizeof(int);
 }
 
 extern __shared__ __align__(16) double rhs_sm[];
@@ -234,8 +237,10 @@ struct RhsBlock {
     long long plane, gij;            // gij: plane offset of the first point
 };
 
-// The march of field F's threads: 0 u, 1 v, 2 w, 3 c.
-template <int ORDER, int MODE, int F, bool EVEN>
+// The march of field F's threads: 0 u, 1 v, 2 w, 3 c.  RCS: the scalars that
+// every row needs wait behind its metrics in shared memory instead of in
+// registers or the constant bank (k_rhs_batch).
+template <int ORDER, int MODE, int F, bool EVEN, bool RCS>
 __device__ __forceinline__ void rhs_field(const Geo& G, const RhsArgs& A, const RhsBlock& T)
 {
     using RT = RhsTile<ORDER>;
@@ -246,7 +251,7 @@ __device__ __forceinline__ void rhs_field(const Geo& G, const RhsArgs& A, const 
     double* __restrict__ fout = (F == 0 ? A.fu : F == 1 ? A.fv : F == 2 ? A.fw : A.fc) + T.gij + T.kb * T.plane;   // row k
     double* gio = A.sw[F].g + T.gij + T.kb * T.plane;                                                             // row k
     double* const mine = rhs_sm + F * RT::FIELD;
-    const int* const goff = reinterpret_cast<const int*>(rhs_sm + rhs_offs<ORDER>());   // plane offsets of the copies
+    const int* const goff = reinterpret_cast<const int*>(rhs_sm + rhs_offs<ORDER, RCS>());   // plane offsets of the copies
     const int at = (T.ty + RT::H) * PJ + T.jl + RT::XL;           // own point within a plane
     const double2 z2 = make_double2(0.0, 0.0);
 
@@ -266,8 +271,8 @@ __device__ __forceinline__ void rhs_field(const Geo& G, const RhsArgs& A, const 
         }
         b += T.plane;
     };
-    double* const cst = rhs_sm + rhs_rows<ORDER>() + F * 2 * (RT_FWMAX + RT_MROW);   // [2][RT_FWMAX] fused coefficients
-    double* const mst = cst + 2 * RT_FWMAX;                      // [2][RT_MROW] grid metrics
+    double* const cst = rhs_sm + rhs_rows<ORDER>() + F * 2 * (RT_FWMAX + RT_MROW<RCS>);   // [2][RT_FWMAX] fused coefficients
+    double* const mst = cst + 2 * RT_FWMAX;                      // [2][RT_MROW<RCS>] grid metrics
     // thread e copies value e of a row: its coefficients, then the metrics
     // (rows kk-1 .. kk+2 lie within 0 .. n2-1)
     const double* xsrc = nullptr;
@@ -282,7 +287,7 @@ __device__ __forceinline__ void rhs_field(const Geo& G, const RhsArgs& A, const 
         xstep = 1;
         xdst = 2 * RT_FWMAX + m;
     }
-    const int xodd = T.q < FWR ? RT_FWMAX : RT_MROW;
+    const int xodd = T.q < FWR ? RT_FWMAX : RT_MROW<RCS>;
     auto load_extras = [&](int kk) {   // (the w solve has nz - 1 rows)
         if (xsrc && !(F == 2 && T.q < FWR && kk >= top)) cp_async8(cst + xdst + (kk & 1) * xodd, xsrc);
         xsrc = xsrc ? xsrc + xstep : xsrc;
@@ -292,6 +297,14 @@ __device__ __forceinline__ void rhs_field(const Geo& G, const RhsArgs& A, const 
         if (EVEN) return T.v0 ? ld2(p) : z2;
         return make_double2(T.v0 ? p[0] : 0.0, T.v1 ? p[1] : 0.0);
     };
+    if (RCS && T.q < 2) {
+        double* c = mst + T.q * RT_MROW<RCS>;
+        c[RM_DXDY] = G.dxdy;
+        c[RM_DIFF] = F == 3 ? A.kappa : A.nu;
+        c[RM_SHIFT] = A.sw[F].gshift ? *A.sw[F].gshift : 0.0;
+        c[RM_IDX2] = G.idx * G.idx;
+        c[RM_IDY2] = G.idy * G.idy;
+    }
     load_extras(T.kb);
     for (int kk = T.kb - RT::ZH; kk <= T.kb + RT::ZH; kk++) load_plane(kk);
     double2 gnext = load_g(T.kb, gio);
@@ -326,7 +339,7 @@ __device__ __forceinline__ void rhs_field(const Geo& G, const RhsArgs& A, const 
     // z fluxes with the halved face velocity m(k): F1(k) = m(k) (q(k) + q(k+1)),
     // F3(k) = m(k+1) (q(k) + q(k+3)); row k needs F1(k), F1(k-1), F3(k), F3(k-3)
     double2 f1 = z2, mz = z2;   // F1(k-1), m(k); F3 of the last rows in this thread's own slots f3q[k & 3]
-    double* const f3q = rhs_sm + rhs_queue<ORDER>() + 2 * threadIdx.x;
+    double* const f3q = rhs_sm + rhs_queue<ORDER, RCS>() + 2 * threadIdx.x;
     double2 kz = z2, fz = z2;                                 // scalar: z curvature of row k, flux of face k-1
     if (F < 3) {
         auto own = [&](int d) { return ld2(ringat(F, T.kb + d)); };
@@ -369,16 +382,17 @@ __device__ __forceinline__ void rhs_field(const Geo& G, const RhsArgs& A, const 
         constexpr bool WALL = decltype(wall_tag)::value;   // rows within two of a wall
         const bool live = F != 2 || !WALL || k < top;      // w has no point on the top wall
         double* const fb = rhs_sm + rhs_faces<ORDER>() + (k & 1) * RF_ALL;
-        const double* mrow = mst + (k & 1) * RT_MROW;
+        const double* mrow = mst + (k & 1) * RT_MROW<RCS>;
         auto DYDZ = [&](int d) { return mrow[1 + d]; };
         auto DXDZ = [&](int d) { return mrow[5 + d]; };
+        auto scalar_of = [&](int m, double v) { return RCS ? mrow[m] : v; };
         // the window moves up one row
 #pragma unroll
         for (int d = 0; d < LO + NZ; d++) zw[d] = zw[d + 1];
         zw[LO + NZ] = ld2(ringat(F, k + NZ));
         auto Z = [&](int d) { return LO + d >= 0 ? zw[LO + d >= 0 ? LO + d : 0] : ld2(ringat(F, k + d)); };
         const double2 q0 = Z(0);
-        const double2 gk = gnext + make_double2(shift, shift);
+        const double2 gk = gnext + make_double2(scalar_of(RM_SHIFT, shift), scalar_of(RM_SHIFT, shift));
         if (k + 1 < T.ke) gnext = load_g(k + 1, gio + T.plane);
 
         // ---- plane k: x neighbours, y neighbours (columns j-4 .. j+5)
@@ -395,21 +409,22 @@ __device__ __forceinline__ void rhs_field(const Geo& G, const RhsArgs& A, const 
             return (e & 1) == 0 ? y[e / 2] : make_double2(y[(e - 1) / 2].y, y[(e + 1) / 2].x);
         };
         // add_laplacexy_operator_{u,w}{2,4} (diffuseu.c:286-359, diffusew.c:290-363)
+        const double rx = scalar_of(RM_IDX2, idx2), ry = scalar_of(RM_IDY2, idy2);
         double2 lap;
         if (ORDER == 2) {
-            lap = idx2 * (X(1) - 2.0 * q0 + X(-1)) + idy2 * (Y(1) - 2.0 * q0 + Y(-1));
+            lap = rx * (X(1) - 2.0 * q0 + X(-1)) + ry * (Y(1) - 2.0 * q0 + Y(-1));
         } else {
-            const double lapc = -2.0 * (L1 + L2 + L3) * (idx2 + idy2);
+            const double lapc = -2.0 * (L1 + L2 + L3) * (rx + ry);
             const double2 lx = L3 * (X(3) + X(-3)) + L2 * (X(2) + X(-2)) + L1 * (X(1) + X(-1));
             const double2 ly = L3 * (Y(3) + Y(-3)) + L2 * (Y(2) + Y(-2)) + L1 * (Y(1) + Y(-1));
-            lap = (idx2 * lx + idy2 * ly) + lapc * q0;
+            lap = (rx * lx + ry * ly) + lapc * q0;
         }
         // the explicit diffusion enters first at order 2 and last at order 4, by measurement (64 x 64 x 384
         // 413 -> 399 us, 256 x 256 x 192 at order 4 the other way round 619 -> 626)
-        if (MODE == RHS_CHANNEL) lap = diff * lap;
+        if (MODE == RHS_CHANNEL) lap = scalar_of(RM_DIFF, diff) * lap;
         auto onto_lap = [&](Product2 advection) -> double2 {
             if (MODE == RHS_CHANNEL || ORDER == 4) return advection;
-            return advection + diff * lap;
+            return advection + scalar_of(RM_DIFF, diff) * lap;
         };
 
         // ---- faces for the other fields, and the flux of the field's own direction
@@ -485,7 +500,7 @@ __device__ __forceinline__ void rhs_field(const Geo& G, const RhsArgs& A, const 
             const Product2 fxm = quick(DYDZ(0) * ld2(u - PJ), X(-1), q0, curv(q0, X(-1), X(-2)), kx0);
             const Product2 fyp = quick(DXDZ(0) * vb, q0, Y(1), ky0, curv(Y(2), Y(1), q0));
             const Product2 fym = quick(DXDZ(0) * make_double2(va.y, vb.x), Y(-1), q0, curv(q0, Y(-1), Y(-2)), ky0);
-            const double2 fzp = quick(dxdy * ld2(ringat(2, k)), q0, Z(1), kz, kzp);
+            const double2 fzp = quick(scalar_of(RM_DXDY, dxdy) * ld2(ringat(2, k)), q0, Z(1), kz, kzp);
             f = onto_lap((-mrow[8]) * ((fxp - fxm) + (fyp - fym) + (fzp - fz)));
             kz = kzp;
             fz = fzp;
@@ -539,9 +554,9 @@ __device__ __forceinline__ void rhs_field(const Geo& G, const RhsArgs& A, const 
                 mz = mup;
             }
             const double2 zs = ORDER == 2 ? zph - zmh : A1 * (zph - zmh) + A2 * (zp3 - zm3);
-            if (F == 0) f = onto_lap((-mrow[8]) * ((DYDZ(0) * own + DXDZ(0) * other) + dxdy * zs));
-            if (F == 1) f = onto_lap((-mrow[8]) * ((DYDZ(0) * other + DXDZ(0) * own) + dxdy * zs));
-            if (F == 2) f = onto_lap((-mrow[9]) * (other + dxdy * zs));
+            if (F == 0) f = onto_lap((-mrow[8]) * ((DYDZ(0) * own + DXDZ(0) * other) + scalar_of(RM_DXDY, dxdy) * zs));
+            if (F == 1) f = onto_lap((-mrow[8]) * ((DYDZ(0) * other + DXDZ(0) * own) + scalar_of(RM_DXDY, dxdy) * zs));
+            if (F == 2) f = onto_lap((-mrow[9]) * (other + scalar_of(RM_DXDY, dxdy) * zs));
             // add_buoyancy{2,4} (scalar.c:6-76); skipped when every betg is zero
             if (buoyancy) {
                 const double* c = ringat(3, k);
@@ -562,7 +577,7 @@ __device__ __forceinline__ void rhs_field(const Geo& G, const RhsArgs& A, const 
                 }
             }
         }
-        if (MODE != RHS_CHANNEL && ORDER == 4) f = f + diff * lap;
+        if (MODE != RHS_CHANNEL && ORDER == 4) f = f + scalar_of(RM_DIFF, diff) * lap;
 
         // ---- right-hand side of the implicit solve, rows GZ .. (u, v, c: nz rows; w: nz - 1 faces)
         const double2* r2 = reinterpret_cast<const double2*>(cst + (k & 1) * RT_FWMAX);
@@ -658,12 +673,12 @@ __device__ __forceinline__ void rhs_field(const Geo& G, const RhsArgs& A, const 
     }
 }
 
-template <int ORDER, int MODE, bool EVEN>
+template <int ORDER, int MODE, bool EVEN, bool RCS>
 __device__ __forceinline__ void rhs_body(const Geo& G, const RhsArgs& A, uint3 bid)
 {
     using RT = RhsTile<ORDER>;
     RhsBlock T;
-    int* goff = reinterpret_cast<int*>(rhs_sm + rhs_offs<ORDER>());
+    int* goff = reinterpret_cast<int*>(rhs_sm + rhs_offs<ORDER, RCS>());
     const int nx = G.nx, ny = G.ny, tid = threadIdx.x;
     T.i0 = bid.y * RT_I;
     T.j0 = bid.x * RT_J;
@@ -691,25 +706,36 @@ __device__ __forceinline__ void rhs_body(const Geo& G, const RhsArgs& A, uint3 b
     // Warp w works on field w mod 4, so that the warps of one of the SM's four
     // schedulers run the same code.  Every field takes the same barriers.
     switch ((tid >> 5) & 3) {
-    case 0: rhs_field<ORDER, MODE, 0, EVEN>(G, A, T); break;
-    case 1: rhs_field<ORDER, MODE, 1, EVEN>(G, A, T); break;
-    case 2: rhs_field<ORDER, MODE, 2, EVEN>(G, A, T); break;
-    default: rhs_field<ORDER, MODE, 3, EVEN>(G, A, T); break;
+    case 0: rhs_field<ORDER, MODE, 0, EVEN, RCS>(G, A, T); break;
+    case 1: rhs_field<ORDER, MODE, 1, EVEN, RCS>(G, A, T); break;
+    case 2: rhs_field<ORDER, MODE, 2, EVEN, RCS>(G, A, T); break;
+    default: rhs_field<ORDER, MODE, 3, EVEN, RCS>(G, A, T); break;
     }
 }
 
 template <int ORDER, int MODE, bool EVEN>
 __global__ void __launch_bounds__(RT_THREADS, 1) k_rhs(Geo G, RhsArgs A)
 {
-    rhs_body<ORDER, MODE, EVEN>(G, A, blockIdx);
+    rhs_body<ORDER, MODE, EVEN, false>(G, A, blockIdx);
 }
 
-template <int ORDER, bool EVEN>
+// Members with partitioned line solves and those without: at order 2 in one
+// launch, FORM_EITHER (of two, the first's last wave runs out before the second
+// begins: 6 flows of 90 x 75 x 53, 100 x 120 x 64 and 240 x 250 x 64, a substep
+// 1372 against 1260 us); at order 4 in launches of their own, since both bodies
+// in one kernel cost more registers than there are (6 x 192 x 192 x 128 a
+// substep 3356 against 3519 us; the mixed sizes above 1683 against 1644).
+// A record's scalars are no constants and cost registers too.  Without the
+// sweep they go to shared memory (RCS), 8 x 128 x 128 x 96 at order 4 a substep 1872 -> 1584
+// us; with it the spills are cheaper, 6 x 192 x 192 x 128 3356 against 3510.
+enum RhsForm { FORM_EITHER, FORM_SWEEP, FORM_H };
+template <int ORDER, int FORM, bool EVEN>
 __global__ void __launch_bounds__(RT_THREADS, 1) k_rhs_batch(const BatchRec<RhsArgs>* r, int n)
 {
     uint3 b;
     const BatchRec<RhsArgs>& R = batch_locate(r, n, b);
-    rhs_body<ORDER, RHS_SWEEP, EVEN>(R.G, R.A, b);
+    if (FORM == FORM_H || (FORM == FORM_EITHER && R.G.partitioned)) rhs_body<ORDER, RHS_H, EVEN, true>(R.G, R.A, b);
+    else rhs_body<ORDER, RHS_SWEEP, EVEN, false>(R.G, R.A, b);
 }
 
 // ------------------------------------------------------------- launchers
@@ -738,12 +764,15 @@ dim3 grid_rhs(const Geo& G, int chunk)
 
 long long rhs_tiles(const Geo& G) { return (long long) ((G.ny + RT_J - 1) / RT_J) * ((G.nx + RT_I - 1) / RT_I); }
 
-// Rows per k_rhs block of an instance that runs alone.  One block fills an
-// SM, so the time is the number of waves times a block's rows plus its
-// start (the ring's first planes and the primed fluxes, about RHS_START
-// rows); the chunk count with the least of it is taken.  Whole columns with
-// the forward sweep in the kernel (sweep), and where the tiles alone give
-// three quarters of the SMs a block (as line_partitioned).
+// Rows per k_rhs block of an instance that has `sms` SMs to itself (in a batch,
+// its share of them by tiles).  One block fills an SM, so the time is the
+// number of waves times a block's rows plus its start (the ring's first planes
+// and the primed fluxes, about RHS_START rows); the chunk count with the least
+// of it is taken.  Whole columns with the forward sweep in the kernel (sweep),
+// and where the tiles alone give three quarters of the SMs a block (as
+// line_partitioned).  Results do not depend on it: a block primes the fluxes
+// and curvatures that it would have carried up, in the same operations
+// (rounding.cuh).
 int rhs_chunk(const Geo& G, int sms, bool sweep)
 {
     constexpr int RHS_START = 4;
@@ -770,17 +799,18 @@ void launch_ghosts_batch(const BatchLaunch& L, int order, cudaStream_t st)
     else k_ghosts_batch<4, true><<<L.blocks, GHOST_THREADS, 0, st>>>(r, L.n);
 }
 
-// (whole columns in a batch: line_partitioned; key: order, + 8 for odd ny)
 void launch_rhs_batch(const BatchLaunch& L, int key, cudaStream_t st)
 {
     auto r = static_cast<const BatchRec<RhsArgs>*>(L.recs);
     const dim3 blk(RT_THREADS);
+#define CASE_(key_, o_, form_) \
+    case key_: k_rhs_batch<o_, form_, true><<<L.blocks, blk, rhs_smem_bytes<o_, true>(), st>>>(r, L.n); break; \
+    case key_ + 8: k_rhs_batch<o_, form_, false><<<L.blocks, blk, rhs_smem_bytes<o_, true>(), st>>>(r, L.n); break;
     switch (key) {
-    case 2: k_rhs_batch<2, true><<<L.blocks, blk, rhs_smem_bytes<2>(), st>>>(r, L.n); break;
-    case 4: k_rhs_batch<4, true><<<L.blocks, blk, rhs_smem_bytes<4>(), st>>>(r, L.n); break;
-    case 10: k_rhs_batch<2, false><<<L.blocks, blk, rhs_smem_bytes<2>(), st>>>(r, L.n); break;
-    default: k_rhs_batch<4, false><<<L.blocks, blk, rhs_smem_bytes<4>(), st>>>(r, L.n); break;
+    CASE_(2, 2, FORM_EITHER) CASE_(4, 4, FORM_SWEEP) CASE_(20, 4, FORM_H)
+    default: break;
     }
+#undef CASE_
 }
 
 void launch_rhs(const Geo& G, const RhsArgs& A, bool implicit3d, cudaStream_t st)
@@ -799,7 +829,7 @@ void launch_rhs(const Geo& G, const RhsArgs& A, bool implicit3d, cudaStream_t st
 
 cudaError_t rhs_set_smem_limits()
 {
-    const int v2 = (int) rhs_smem_bytes<2>(), v4 = (int) rhs_smem_bytes<4>();
+    const int v2 = (int) rhs_smem_bytes<2, true>(), v4 = (int) rhs_smem_bytes<4, true>();
     cudaError_t e = cudaSuccess;
     auto set = [&](const void* f, int v) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
@@ -816,10 +846,12 @@ cudaError_t rhs_set_smem_limits()
     set((const void*) k_rhs<4, RHS_H, false>, v4);
     set((const void*) k_rhs<4, RHS_CHANNEL, true>, v4);
     set((const void*) k_rhs<4, RHS_CHANNEL, false>, v4);
-    set((const void*) k_rhs_batch<2, true>, v2);
-    set((const void*) k_rhs_batch<2, false>, v2);
-    set((const void*) k_rhs_batch<4, true>, v4);
-    set((const void*) k_rhs_batch<4, false>, v4);
+    set((const void*) k_rhs_batch<2, FORM_EITHER, true>, v2);
+    set((const void*) k_rhs_batch<2, FORM_EITHER, false>, v2);
+    set((const void*) k_rhs_batch<4, FORM_SWEEP, true>, v4);
+    set((const void*) k_rhs_batch<4, FORM_SWEEP, false>, v4);
+    set((const void*) k_rhs_batch<4, FORM_H, true>, v4);
+    set((const void*) k_rhs_batch<4, FORM_H, false>, v4);
     return e;
 }
 

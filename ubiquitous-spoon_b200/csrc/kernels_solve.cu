@@ -523,13 +523,12 @@ __global__ void __launch_bounds__(CHUNKS ? 256 : 128, CHUNKS ? 2 : 9) k_line(Geo
     line_body<ORDER, CHUNKS>(G, B, blockIdx);
 }
 
-// (whole columns in a batch: line_partitioned)
-template <int ORDER>
-__global__ void __launch_bounds__(128, 9) k_line_batch(const BatchRec<SolveBatch>* r, int n)
+template <int ORDER, bool CHUNKS>
+__global__ void __launch_bounds__(CHUNKS ? 256 : 128, CHUNKS ? 2 : 9) k_line_batch(const BatchRec<SolveBatch>* r, int n)
 {
     uint3 b;
     const BatchRec<SolveBatch>& R = batch_locate(r, n, b);
-    line_body<ORDER, false>(R.G, R.A, b);
+    line_body<ORDER, CHUNKS>(R.G, R.A, b);
 }
 
 // Threads of a block, from the tuned solve_threads: at C chunks, the groups of
@@ -539,7 +538,16 @@ int line_threads(const Geo& G)
 {
     if (!G.partitioned) return G.shape.solve_threads;
     const int C = line_chunk_count(G.nz);
-    return std::max(1, (G.shape.solve_threads == 64 ? 96 : 192) / (8 * C)) * 8 * C;
+    return std::max(1, line_batch_threads(G) / (8 * C)) * 8 * C;
+}
+
+// Threads of a batched launch's blocks, the same for every member's C; those
+// beyond a member's line_threads have no chunk.
+int line_batch_threads(const Geo& G)
+{
+    if (!G.partitioned) return G.shape.solve_threads;
+    static_assert(8 * line_chunk_count(LINE_MAX_ROWS) <= 96, "a group of columns of the tallest member fits");
+    return G.shape.solve_threads == 64 ? 96 : 192;
 }
 
 dim3 grid_line(const Geo& G)
@@ -589,11 +597,15 @@ void launch_mass_control(const MassArgs& M, cudaStream_t st)
     k_mass_control<<<1, 32, 0, st>>>(M);
 }
 
-void launch_line_batch(const BatchLaunch& L, int order, cudaStream_t st)
+void launch_line_batch(const BatchLaunch& L, int key, cudaStream_t st)
 {
     auto r = static_cast<const BatchRec<SolveBatch>*>(L.recs);
-    if (order == 2) k_line_batch<2><<<L.blocks, L.block, 0, st>>>(r, L.n);
-    else k_line_batch<4><<<L.blocks, L.block, 0, st>>>(r, L.n);
+    switch (key) {
+    case 2: k_line_batch<2, false><<<L.blocks, L.block, 0, st>>>(r, L.n); break;
+    case 4: k_line_batch<4, false><<<L.blocks, L.block, 0, st>>>(r, L.n); break;
+    case 18: k_line_batch<2, true><<<L.blocks, L.block, L.smem, st>>>(r, L.n); break;
+    default: k_line_batch<4, true><<<L.blocks, L.block, L.smem, st>>>(r, L.n); break;
+    }
 }
 
 void launch_control_batch(const BatchLaunch& L, cudaStream_t st)
