@@ -321,12 +321,14 @@ __device__ __forceinline__ void line_chunks(const Geo& G, const SolveArgs& A, ui
 // The back sweep with one thread per column, of rows whose forward sweep k_rhs
 // has done (its SWEEP variant); s of row i - PD is loaded while row i is
 // computed.
-// Bound: HBM, 16 bytes per point and field; 1.47 ms for four fields at
-// 512 x 512 x 384 (4.4 TB/s).
+// Bound: HBM, 16 bytes per point and field; 1.08 ms for four fields at
+// 512 x 512 x 384, order 4 (6.0 TB/s).  That takes about 70 KB of loads in flight
+// on an SM: PD = 8 at 9 or 10 blocks.  With PD = 4, us for the four fields,
+// 512 x 512 x 384 order 4 1480, 300 x 320 x 200 order 2 312 (now 226).
 template <int ORDER, bool IS_W, bool STATS>
 __device__ __forceinline__ void back_column(const Geo& G, const SolveArgs& A, uint3 bid)
 {
-    constexpr int H = ORDER == 2 ? 1 : 3, PD = 4;
+    constexpr int H = ORDER == 2 ? 1 : 3, PD = 8;
     const long long P = G.plane, col = (long long) bid.x * blockDim.x + threadIdx.x;
     const bool valid = col < P;
     const int n = A.n, n2 = G.n2;
@@ -356,6 +358,7 @@ __device__ __forceinline__ void back_column(const Geo& G, const SolveArgs& A, ui
     // they would cost resident blocks)
     auto again = [&](int i) { return valid && i >= 0 ? x[(GZ + i) * P] : 0.0; };
     const double top0 = again(n - 1), top1 = again(n - 2), top2 = again(n - 3);
+    const double mid0 = STATS ? again((G.nz - 1) / 2) : 0.0, mid1 = STATS ? again(G.nz / 2) : 0.0;
     double gb1, gb2, gt1, gt2;
     ghosts_bot<ORDER, IS_W>(A, x, P, valid, y1, y2, y3, gb1, gb2);
     ghosts_top<ORDER, IS_W>(A, x, P, n2, valid, top0, top1, top2, gt1, gt2);
@@ -374,8 +377,8 @@ __device__ __forceinline__ void back_column(const Geo& G, const SolveArgs& A, ui
     put(6, top0);
     put(7, gt1);
     put(8, gt2);
-    put(9, again((G.nz - 1) / 2));
-    put(10, again(G.nz / 2));
+    put(9, mid0);
+    put(10, mid1);
 }
 
 // The control and its log row from the bulk mean, the averages of rows
@@ -515,16 +518,21 @@ __device__ __forceinline__ void line_body(const Geo& G, const SolveBatch& B, uin
     }
 }
 
-// The back sweep: nine blocks of 128 threads per SM (56 registers); one
-// fewer measured 40 % slower.
+// Blocks of 128 threads per SM of the back sweep.  Order 4: 56 registers, one block
+// fewer measured 45 % slower at 512 x 512 x 384; order 2: 48 registers, 512 x 512
+// x 256 665 us, with 9 blocks 946, with 12 (40 registers) 849.  The batched form
+// of order 4 takes 10 (3 x 256 x 256 x 192, a substep 4167 us, with 9 4246).
+template <int ORDER>
+constexpr int BACK_BLOCKS = ORDER == 2 ? 10 : 9;
+
 template <int ORDER, bool CHUNKS>
-__global__ void __launch_bounds__(CHUNKS ? 256 : 128, CHUNKS ? 2 : 9) k_line(Geo G, SolveBatch B)
+__global__ void __launch_bounds__(CHUNKS ? 256 : 128, CHUNKS ? 2 : BACK_BLOCKS<ORDER>) k_line(Geo G, SolveBatch B)
 {
     line_body<ORDER, CHUNKS>(G, B, blockIdx);
 }
 
 template <int ORDER, bool CHUNKS>
-__global__ void __launch_bounds__(CHUNKS ? 256 : 128, CHUNKS ? 2 : 9) k_line_batch(const BatchRec<SolveBatch>* r, int n)
+__global__ void __launch_bounds__(CHUNKS ? 256 : 128, CHUNKS ? 2 : 10) k_line_batch(const BatchRec<SolveBatch>* r, int n)
 {
     uint3 b;
     const BatchRec<SolveBatch>& R = batch_locate(r, n, b);
