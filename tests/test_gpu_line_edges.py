@@ -5,6 +5,11 @@ and the packed x transforms change form, against the numpy restatement:
   of one row (where w, one row shorter, has none), the tallest partitioned
   column (192 rows) and the first whole-column one (193);
 * planes whose columns do not fill the last group of 16 (or of 32), odd and even;
+* whole columns of even planes at both orders, by their height (193 rows, several
+  partial tiles) and by their plane (more than 111 tiles), fewer rows than the back
+  sweep reads ahead;
+* rows that k_rhs's blocks do not divide: last blocks of one row and of two, in both
+  schemes;
 * x transforms of two columns each: an odd last column, 16-column blocks with
   one column and with fifteen;
 * transforms planned at run time: one stage (4, 5), the largest size (500),
@@ -21,6 +26,7 @@ import pytest
 
 import chanfast_np as cn
 import ic
+from perf import cases
 
 pytestmark = pytest.mark.gpu
 
@@ -30,7 +36,12 @@ TRANSFORMS = [(2, 500, 4, 4), (4, 5, 500, 6), (2, 4, 486, 5), (4, 243, 8, 6), (2
               (4, 48, 18, 7), (2, 192, 30, 5), (4, 192, 9, 6), (4, 320, 15, 6)]
 
 
-@pytest.mark.parametrize("order,nx,ny,nz", CASES + TRANSFORMS)
+WHOLE = [(2, 40, 72, 193), (4, 40, 72, 193), (2, 200, 160, 9), (4, 200, 160, 9), (2, 200, 160, 4)]
+# on 148 SMs blocks of 7 rows and a last one of 1 (43) or 2 (37)
+SHORT_BLOCKS = [(2, 64, 64, 43), (4, 64, 64, 43), (2, 64, 64, 37), (4, 64, 64, 37)]
+
+
+@pytest.mark.parametrize("order,nx,ny,nz", CASES + TRANSFORMS + WHOLE + SHORT_BLOCKS)
 def test_substeps_match_restatement(cf, gpu, order, nx, ny, nz):
     prm = cn.Params(order=order, nx=nx, ny=ny, nz=nz, lx=2 * np.pi, ly=np.pi, lz=2.0, dt=1e-3, nu=1.0 / 3000.0,
                     prandtl=0.71, setuframe=0.3, betg_x=0.1, betg_y=0.05, betg_z=0.02)
@@ -54,6 +65,22 @@ def test_substeps_match_restatement(cf, gpu, order, nx, ny, nz):
         bar = 1e-9 * np.maximum(np.abs(ref).max(axis=0), 1e-3)
         bar[[0, 5]] = np.maximum(bar[[0, 5]], 1e-14 / prm.dt)
         assert np.all(np.abs(log - ref) <= bar), np.abs(log - ref).max(axis=0)
+
+
+@pytest.mark.parametrize("order,nz", [(2, 43), (4, 43), (2, 37), (4, 37)])
+def test_fully_implicit_scheme_with_short_blocks(cf, gpu, order, nz):
+    """Its right-hand side takes the same row blocks: against the plain 64-bit
+    torch statement of the scheme.  Bars as test_gpu_channel.py: 1e-12 on
+    u, v, w, c and 1e-10 on p."""
+    case = cases.flow("short", "step", order, 64, 64, nz, 1, scheme="channel", re=100.0, dt=1e-3, betg=0.1, uframe=0.3)
+    state = cases.prepare(case, 5)
+    got = cases.run(state)
+    state["inst"].sync()
+    want = cases.exact(case, 5)
+    for nm in "uvwcp":
+        rel = float((got[nm] - want[nm]).norm() / want[nm].norm())
+        assert rel <= (1e-10 if nm == "p" else 1e-12), (nm, rel)
+    state["inst"].close()
 
 
 def test_batch_of_odd_and_even_planes_matches_plain(cf, gpu):

@@ -3,8 +3,8 @@
 The tuned kernels index their work from blockDim, one column, column pair or
 point per thread, so every candidate shape must give the same results bit
 for bit; the tuner may then pick any of them.  Cases include planes that are
-not a multiple of the block size (padding warps in the per-warp row sums of
-the back substitution) and both orders."""
+not a multiple of the block size (padding lanes and warps in the line solves'
+column sums), partitioned and whole columns (193 rows), and both orders."""
 import os
 import subprocess
 import sys
@@ -44,7 +44,8 @@ def test_tuned_shape_is_a_candidate_and_cached(cf, gpu):
             a.set_launch_shape((128, 128, 16, 4))
 
 
-@pytest.mark.parametrize("order,nx,ny,nz", [(2, 48, 40, 16), (4, 96, 72, 24), (4, 128, 128, 32)])
+@pytest.mark.parametrize("order,nx,ny,nz", [(2, 48, 40, 16), (4, 96, 72, 24), (4, 128, 128, 32), (2, 10, 9, 193),
+                                              (4, 10, 9, 193), (2, 48, 40, 193), (4, 48, 40, 193)])
 def test_every_shape_gives_identical_results(cf, gpu, order, nx, ny, nz):
     c = cfg(cf, order, nx, ny, nz)
     out = []
