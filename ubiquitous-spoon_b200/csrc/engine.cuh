@@ -274,7 +274,7 @@ cudaError_t fft_set_smem_limits();
 struct BatchLaunch;
 dim3 grid_ghosts(const Geo& G);
 dim3 grid_rhs(const Geo& G, int chunk);
-constexpr int RHS_MIN_ROWS = 6;      // fewest rows of a k_rhs block (its wall closures reach two rows)
+constexpr int RHS_MIN_ROWS = 6;      // fewest rows that rhs_chunk gives a k_rhs block; a column's last block takes what is left, down to one row
 long long rhs_tiles(const Geo& G);
 int rhs_chunk(const Geo& G, int sms, bool sweep);
 int line_threads(const Geo& G);

@@ -454,7 +454,7 @@ __global__ void k_mass_control(MassArgs A)
 // fixed order, and the last block to finish does both controls.  One launch
 // of 2 x LINE_STATS blocks in place of four (two row averages over n2 rows of
 // every 32 columns, two single-block controls): 7 against 17 us at
-// 64 x 64 x 64, 10 against 56 us at 512 x 512 x 384, where it reads 0.7 MB of
+// 64 x 64 x 64, 10 against 56 us at 512 x 512 x 384, where it reads 1.4 MB of
 // sums instead of 51 MB.
 __device__ __forceinline__ void control_body(const ControlArgs& A, uint3 bid)
 {
