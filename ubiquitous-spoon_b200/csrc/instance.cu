@@ -472,14 +472,16 @@ namespace {
 // partition is for planes too small to give every SM a k_rhs tile: k_rhs then
 // gets its blocks from the rows, and k_line's threads walk 16 rows instead of
 // all.  Measured, k_rhs + k_line in us, partitioned against whole columns:
-//   order 2: 64^3 30 : 100, 128 x 128 x 96 96 : 162, 192 x 192 x 128 250 : 258
-//   order 4: 64^3 40 : 157, 128 x 128 x 96 136 : 241, 192 x 192 x 128 339 : 334
+//   order 2: 64^3 30 : 100, 128 x 128 x 96 94 : 162, 192 x 192 x 128 250 : 225
+//   order 4: 64^3 41 : 157, 128 x 128 x 96 126 : 241, 192 x 192 x 128 339 : 290
 // The line lies at three quarters of the SMs (192 x 192 has 144 tiles): from
 // there on the row blocks' start costs what the idle SMs cost, and work on
 // other streams, which fills those, is slowed (256 x 256 x 192 at order 4,
-// three instances at once: 8.54 against 8.32 ms).  Above 192 rows the carries
-// through the chunks cost more than the walk (512 x 512 x 384: 2880 against
-// 1480 us).
+// three instances at once: 8.54 against 8.32 ms).  Above 192 rows a group of
+// columns no longer fits the smaller block of k_line (96 threads); how tall
+// columns of small planes would fare partitioned is not measured (64 x 64 x 384
+// whole: order 2 498 us, order 4 752).  On large planes the partition loses:
+// 512 x 512 x 384, order 4, k_line 2880 against 1085 us.
 bool line_partitioned(bool channel, const Geo& G, int sms)
 {
     return !channel && G.nz <= LINE_MAX_ROWS && 4 * rhs_tiles(G) <= 3 * sms;

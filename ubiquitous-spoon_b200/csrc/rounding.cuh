@@ -11,7 +11,7 @@
 namespace cf {
 
 __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ double add(double a, double b) { return a + b; }   // no product to fuse: mul is opaque to the compiler
 __device__ __forceinline__ double mad(double a, double b, double c) { return __fma_rn(a, b, c); }    // c + a b
 __device__ __forceinline__ double msub(double a, double b, double c) { return __fma_rn(-a, b, c); }  // c - a b
 // a x + b y (+ c z + ...)
