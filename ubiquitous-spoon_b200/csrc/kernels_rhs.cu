@@ -107,12 +107,12 @@ __global__ void k_ghosts_batch(const BatchRec<GhostArgs>* r, int n)
 // block-wide barrier per row is enough.
 //
 // Bound: instruction issue and shared-memory bandwidth (order 4, ncu at
-// 256 x 256 x 192: LSU wavefronts 69 %, FP64 41 %, issue 54 %).  One thread
+// 256 x 256 x 192: LSU wavefronts 70 %, FP64 42 %, issue 52 %).  One thread
 // per point doing all four equations (256 threads, 253 registers) formed each
 // interpolated velocity four times and had two warps per scheduler to hide
-// latency with.  us, before and now: order 4 512 x 512 x 384 5161 -> 4390,
-// 256 x 256 x 192 748 -> 633, 128 x 128 x 96 (row blocks) 99 -> 89; order 2
-// 256 x 256 x 192 507 -> 478, 192 x 192 x 128 179 -> 168.
+// latency with.  us, before and now: order 4 512 x 512 x 384 5161 -> 4174,
+// 256 x 256 x 192 748 -> 621, 128 x 128 x 96 (row blocks) 99 -> 89; order 2
+// 256 x 256 x 192 507 -> 480, 128 x 128 x 96 (row blocks) 66.
 // The four equations' loops have to fit the SM's instruction cache together
 // (about 27 KB at order 4): with two rows of points a thread, fewer
 // instructions but 42 KB of code, the warps waited for instructions (1105 us at
@@ -124,7 +124,9 @@ __global__ void k_ghosts_batch(const BatchRec<GhostArgs>* r, int n)
 // Divisions by the grid metrics are multiplications by their reciprocals (host
 // tables), the 0.5 of a face average is folded into the interpolation weights
 // and a direction's metric is factored out of its flux sum, so results agree
-// with the reference to rounding, not bit for bit.
+// with the reference to rounding, not bit for bit.  Which product of a sum is
+// fused is written down (rounding.cuh): the same flow in another instantiation
+// of the body, or in other row blocks, gives the same bits.
 //
 // After a row's explicit right-hand side the thread forms the right-hand side
 // h of its implicit solve (chanfast.c:459-480), which overwrites g.
